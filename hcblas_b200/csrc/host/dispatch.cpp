@@ -32,6 +32,16 @@ bool aligned16(const void *p, int64_t off, int esz) {
   return ((reinterpret_cast<uintptr_t>(p) + (uintptr_t)(off * esz)) & 15) == 0;
 }
 
+/* M N K from which HGEMM with operands that TMA cannot address copies them
+ * into addressable scratch and runs on the tensor cores instead of the CUDA
+ * cores.  Measured (B200, CUDA-core kernel against copy + tensor cores):
+ * 645 x 645 x 647 37 against 18 us, 1133 x 777 x 1133 105 against 22,
+ * 8378 x 32 x 1024 48 against 23, 8191 x 4095 x 17 109 against 53,
+ * 8378 x 1133 x 777 521 against 51 (beta != 0), 4095^3 3416 against 139.
+ * Smaller products keep the path that needs neither scratch nor a second
+ * launch. */
+constexpr double REALIGN_MIN_MNK = 268435456.0; /* 2^28 */
+
 int simt(HcblasB200State *st, const hcbk_gemm_args *a, void *stream, const char **path) {
   if (a->dtype == HCBK_D && st->dgemm_dmma) {
     /* native FP64 on the DMMA path (mma.sync .f64) */
@@ -82,12 +92,51 @@ bool use_pair(const HcblasB200State *st, int64_t m, int64_t n, int64_t bn) {
   return tiles_of(m, n, 256, bn) >= hcbk_sm_count() / 2;
 }
 
-/* HGEMM on tcgen05 with operands read in place by TMA. */
+/* HGEMM on tcgen05 with operands read in place by TMA; an operand that TMA
+ * cannot address (base or leading dimension off 16 bytes) is first copied
+ * into scratch lines that it can, when the product is large enough to pay for
+ * the extra pass and launch. */
 int hgemm_tc(HcblasB200State *st, const hcbk_gemm_args *a, void *stream, const char **path) {
   if (a->batch != 1 || a->a_array) return HCBK_ERR_ARGS;
-  if (!aligned16(a->a, a->a_off, 2) || !aligned16(a->b, a->b_off, 2) || (a->lda & 7) ||
-      (a->ldb & 7))
-    return HCBK_ERR_ALIGN;
+  const bool ok_a = aligned16(a->a, a->a_off, 2) && !(a->lda & 7);
+  const bool ok_b = aligned16(a->b, a->b_off, 2) && !(a->ldb & 7);
+  if (!ok_a || !ok_b) {
+    if (st->inject_timeout || (double)a->m * (double)a->n * (double)a->k < REALIGN_MIN_MNK ||
+        a->m > 0x7fffffff || a->n > 0x7fffffff || a->k > 0x7fffffff)
+      return HCBK_ERR_ALIGN;
+    /* stored lines: `inner` contiguous elements, `outer` lines */
+    const int64_t in_a = a->op_a == HCBK_OP_N ? a->m : a->k;
+    const int64_t out_a = a->op_a == HCBK_OP_N ? a->k : a->m;
+    const int64_t in_b = a->op_b == HCBK_OP_N ? a->k : a->n;
+    const int64_t out_b = a->op_b == HCBK_OP_N ? a->n : a->k;
+    auto up8 = [](int64_t v) { return (v + 7) & ~int64_t(7); };
+    const size_t bytes_a = ok_a ? 0 : ((size_t)up8(in_a) * out_a * 2 + 255) & ~size_t(255);
+    const size_t bytes_b = ok_b ? 0 : (size_t)up8(in_b) * out_b * 2;
+    char *ws = static_cast<char *>(call_scratch(st, bytes_a + bytes_b, stream));
+    if (!ws) return HCBK_ERR_ALIGN;
+    hcbk_gemm_args r = *a;
+    hcbk_realign_job jobs[2];
+    int count = 0;
+    if (!ok_a) {
+      jobs[count++] = {static_cast<const uint16_t *>(a->a) + a->a_off, a->lda, ws, up8(in_a),
+                       in_a, out_a};
+      r.a = ws;
+      r.a_off = 0;
+      r.lda = up8(in_a);
+    }
+    if (!ok_b) {
+      jobs[count++] = {static_cast<const uint16_t *>(a->b) + a->b_off, a->ldb, ws + bytes_a,
+                       up8(in_b), in_b, out_b};
+      r.b = ws + bytes_a;
+      r.b_off = 0;
+      r.ldb = up8(in_b);
+    }
+    int rc = timed_launch(st, stream, "pack.realign_f16",
+                          [&] { return hcbk_realign_f16(jobs, count, stream); });
+    if (!rc) rc = hgemm_tc(st, &r, stream, path);
+    call_scratch_free(ws, stream);
+    return rc;
+  }
   int *err = device_error_flag(st);
   if (!err) return HCBK_ERR_NOMEM;
   if (st->inject_timeout) { /* failure-detection test: one call, then disarmed */

@@ -78,7 +78,9 @@ int dispatch_with_graph(HcblasB200State *st, const hcbk_gemm_args *a, void *stre
     return HCBK_OK;
   }
   const char *p2 = nullptr;
+  st->own_capture = stream;
   const int rc2 = dispatch_gemm(st, a, stream, &p2);
+  st->own_capture = nullptr;
   cudaGraph_t graph = nullptr;
   const cudaError_t ce = cudaStreamEndCapture(cs, &graph);
   const long long captured = launch_count() - before;

@@ -113,6 +113,52 @@ void *ensure_workspace(HcblasB200State *st, size_t bytes, void *stream_v) {
   return p;
 }
 
+void *call_scratch(HcblasB200State *st, size_t bytes, void *stream_v) {
+  cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
+  if (st->workspace_limit && bytes > st->workspace_limit) return nullptr;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 16) return nullptr;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream, &cap) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  if (cap != cudaStreamCaptureStatusNone && (!stream_v || st->own_capture != stream_v))
+    return nullptr;
+  cudaMemPool_t pool;
+  {
+    std::lock_guard<std::mutex> lock(st->scratch_mutex);
+    if (!st->scratch_pool[dev]) {
+      cudaMemPoolProps props;
+      std::memset(&props, 0, sizeof(props));
+      props.allocType = cudaMemAllocationTypePinned;
+      props.location.type = cudaMemLocationTypeDevice;
+      props.location.id = dev;
+      cudaMemPool_t made = nullptr;
+      unsigned long long keep = 512ull << 20;
+      if (cudaMemPoolCreate(&made, &props) != cudaSuccess ||
+          cudaMemPoolSetAttribute(made, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+        cudaGetLastError();
+        if (made) cudaMemPoolDestroy(made);
+        return nullptr;
+      }
+      st->scratch_pool[dev] = made;
+    }
+    pool = static_cast<cudaMemPool_t>(st->scratch_pool[dev]);
+  }
+  void *p = nullptr;
+  if (cudaMallocFromPoolAsync(&p, bytes, pool, stream) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  return p;
+}
+
+void call_scratch_free(void *p, void *stream) {
+  if (p && cudaFreeAsync(p, static_cast<cudaStream_t>(stream)) != cudaSuccess) cudaGetLastError();
+}
+
 void clear_graph_cache(HcblasB200State *st) {
   for (auto &e : st->graph_cache)
     if (e.exec) cudaGraphExecDestroy(static_cast<cudaGraphExec_t>(e.exec));
@@ -337,6 +383,13 @@ Hcblaslibrary::~Hcblaslibrary() {
       }
       if (gp.staging) cudaFreeHost(gp.staging);
     }
+    /* memory still in use by queued work is released when that work ends */
+    for (int d = 0; d < 16; ++d)
+      if (impl->scratch_pool[d]) {
+        DeviceGuard g(d);
+        if (cudaMemPoolDestroy(static_cast<cudaMemPool_t>(impl->scratch_pool[d])) != cudaSuccess)
+          cudaGetLastError();
+      }
     delete impl;
     impl = nullptr;
   }

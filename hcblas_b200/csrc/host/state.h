@@ -9,6 +9,7 @@
 #include <stddef.h>
 #include <stdint.h>
 
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -82,6 +83,11 @@ struct HcblasB200State {
   void *workspace_stream = nullptr; /* stream of the last call that used it */
   void *workspace_event = nullptr;  /* cudaEvent_t ordering a new stream after it */
   size_t workspace_limit = 0;       /* tuning knob "workspace_mb" (0 = none) */
+  /* per-device memory pools of call_scratch (created on first use) */
+  std::mutex scratch_mutex;
+  void *scratch_pool[16] = {nullptr}; /* cudaMemPool_t */
+  /* the stream whose calls the library itself is capturing (graphs knob) */
+  void *own_capture = nullptr;
   /* device error block of the tensor-core kernels: int 0 is set when a
    * pipeline wait times out, ints 2-3 hold the wait limit in ns */
   int *dev_err = nullptr;
@@ -167,6 +173,17 @@ class DeviceGuard {
  * `stream` is being captured, beyond the "workspace_mb" limit, or when the
  * allocation fails. */
 void *ensure_workspace(HcblasB200State *st, size_t bytes, void *stream);
+
+/* Scratch memory of one call: allocated stream-ordered from the handle's own
+ * pool and handed back with call_scratch_free after the call's last launch, so
+ * calls on different streams (or from different threads) never share a buffer
+ * and never wait for one another.  The pool keeps up to 512 MiB between calls
+ * and is given back with the handle.  nullptr while the caller captures
+ * `stream` (the memory would belong to the caller's graph), beyond the
+ * "workspace_mb" limit, or when the allocation fails: the caller then takes a
+ * path that needs no scratch. */
+void *call_scratch(HcblasB200State *st, size_t bytes, void *stream);
+void call_scratch_free(void *p, void *stream);
 
 /* The handle's device error flag on the current device (allocated and
  * zeroed on first use); nullptr if it cannot be allocated. */

@@ -114,6 +114,20 @@ int hcbk_hgemm_tc(const hcbk_gemm_args *args, int bn, int pair, int *err, void *
  * when the kernel unwinds.  HCBK_ERR_ARGS for any other shape. */
 int hcbk_hgemm_tc_inject_timeout(const hcbk_gemm_args *args, int *err, void *stream);
 
+/* Copy f16 operands whose lines TMA cannot address (base or leading
+ * dimension off 16 bytes) into lines that it can: line i (`inner` contiguous
+ * elements at src + i * ld) goes to dst + i * ld_dst, ld_dst >= inner a
+ * multiple of 8 and dst 16-byte aligned; the padding is zeroed.  One launch
+ * for one or two operands (count). */
+typedef struct hcbk_realign_job {
+  const void *src;
+  int64_t ld;
+  void *dst;
+  int64_t ld_dst;
+  int64_t inner, outer;
+} hcbk_realign_job;
+int hcbk_realign_f16(const hcbk_realign_job *jobs, int count, void *stream);
+
 /* Split-BF16 SGEMM: operands already split into bf16 planes, K-major:
  * a_planes[t] is M rows x ld_a elements (row m holds op(A)(m, 0..K-1)),
  * b_planes[t] is N rows x ld_b elements (row n holds op(B)(0..K-1, n)).

@@ -203,6 +203,66 @@ __global__ void c3m_combine_kernel(hcbk_c3m_combine_args a) {
   }
 }
 
+/* --------------------------------------------- f16 realignment (HGEMM) -- */
+
+/* Bound by memory: reads and writes the operand once (2 bytes each way per
+ * element).  A warp takes RA_LINES consecutive lines' 256-element segment, 8
+ * elements (one 16-byte store) per lane and line, read as aligned 4-byte
+ * words -- a 4-byte word holding an element of the line is always inside the
+ * allocation -- and shifted by 2 bytes where the line starts at an odd
+ * element.  The RA_LINES independent loads per lane cover the DRAM latency. */
+constexpr int RA_LINES = 4;
+
+struct RealignArgs {
+  hcbk_realign_job j[2];
+  int64_t segs[2];   /* 256-element segments per line */
+  int64_t units[2];  /* warp units of each operand */
+};
+
+__device__ __forceinline__ uint4 load8_f16(const uint16_t *s, int valid) {
+  if (valid >= 8) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(s);
+    const uint32_t *w = reinterpret_cast<const uint32_t *>(at & ~uintptr_t(3));
+    const uint32_t w0 = w[0], w1 = w[1], w2 = w[2], w3 = w[3];
+    if ((at & 2) == 0) return make_uint4(w0, w1, w2, w3);
+    const uint32_t w4 = w[4]; /* its low half is element 7 */
+    return make_uint4(__funnelshift_r(w0, w1, 16), __funnelshift_r(w1, w2, 16),
+                      __funnelshift_r(w2, w3, 16), __funnelshift_r(w3, w4, 16));
+  }
+  uint32_t v[4] = {0u, 0u, 0u, 0u};
+#pragma unroll
+  for (int e = 0; e < 8; ++e)
+    if (e < valid) v[e >> 1] |= (uint32_t)s[e] << (16 * (e & 1));
+  return make_uint4(v[0], v[1], v[2], v[3]);
+}
+
+__global__ void __launch_bounds__(256) realign_f16_kernel(const __grid_constant__ RealignArgs a) {
+  const int lane = threadIdx.x & 31;
+  const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
+  const int64_t total = a.units[0] + a.units[1];
+  for (int64_t u = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); u < total;
+       u += warps) {
+    const int w = u >= a.units[0] ? 1 : 0;
+    const hcbk_realign_job &j = a.j[w];
+    const int64_t x = u - (w ? a.units[0] : 0);
+    const int64_t band = x / a.segs[w];
+    const int64_t e = (x - band * a.segs[w]) * 256 + lane * 8;
+    if (e >= j.ld_dst) continue;
+    const int valid = (int)(j.inner - e < 8 ? j.inner - e : 8);
+    const int64_t l0 = band * RA_LINES;
+    const int lines = (int)(j.outer - l0 < RA_LINES ? j.outer - l0 : RA_LINES);
+    const uint16_t *s = static_cast<const uint16_t *>(j.src) + l0 * j.ld + e;
+    uint16_t *d = static_cast<uint16_t *>(j.dst) + l0 * j.ld_dst + e;
+    uint4 v[RA_LINES];
+#pragma unroll
+    for (int i = 0; i < RA_LINES; ++i)
+      if (i < lines) v[i] = load8_f16(s + i * j.ld, valid);
+#pragma unroll
+    for (int i = 0; i < RA_LINES; ++i)
+      if (i < lines) *reinterpret_cast<uint4 *>(d + i * j.ld_dst) = v[i];
+  }
+}
+
 }  // namespace
 
 extern "C" int hcbk_pack_split_bf16_complex(const hcbk_cpack_args *a, void *stream) {
@@ -287,4 +347,24 @@ extern "C" int hcbk_pack_split_bf16_pair(const hcbk_pack_args *a, const hcbk_pac
   int rc = a->k_contig ? launch_kcontig(&a, 1, st) : launch_rcontig(a, st);
   if (rc) return rc;
   return b->k_contig ? launch_kcontig(&b, 1, st) : launch_rcontig(b, st);
+}
+
+extern "C" int hcbk_realign_f16(const hcbk_realign_job *jobs, int count, void *stream) {
+  if (count < 1 || count > 2) return HCBK_ERR_ARGS;
+  RealignArgs a;
+  memset(&a, 0, sizeof(a));
+  for (int i = 0; i < count; ++i) {
+    const hcbk_realign_job &j = jobs[i];
+    if (j.inner <= 0 || j.outer <= 0 || j.ld_dst < j.inner || (j.ld_dst & 7) ||
+        (reinterpret_cast<uintptr_t>(j.src) & 1) || (reinterpret_cast<uintptr_t>(j.dst) & 15))
+      return HCBK_ERR_ARGS;
+    a.j[i] = j;
+    a.segs[i] = (j.ld_dst + 255) / 256;
+    a.units[i] = a.segs[i] * ((j.outer + RA_LINES - 1) / RA_LINES);
+  }
+  int64_t blocks = (a.units[0] + a.units[1] + 7) / 8;
+  const int64_t most = (int64_t)hcbk_sm_count() * 8;
+  if (blocks > most) blocks = most;
+  realign_f16_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
+  return cudaGetLastError() == cudaSuccess ? HCBK_OK : HCBK_ERR_LAUNCH;
 }

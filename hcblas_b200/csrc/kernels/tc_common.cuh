@@ -23,6 +23,7 @@
 #define HCBLAS_B200_TC_COMMON_CUH_
 
 #include <cuda.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -501,6 +502,147 @@ struct RecipeBf16x6 {
   __host__ __device__ static constexpr int pacc(int i) { return i == 5 ? 0 : 1; }
   __host__ __device__ static constexpr bool first(int i) { return i == 0 || i == 5; }
 };
+
+/* ------------------------------------- f16 C that TMA cannot address -- */
+
+/* An f16 C whose rows or leading dimension are not whole 16-byte chunks.  The
+ * kernel computes the transposed product, so that a TMEM lane is a column of C
+ * and its TMEM columns are consecutive rows: two rows convert to one word in
+ * one instruction, and a warp's 32 columns go through its own part of shared
+ * memory, 128 rows at a time, without meeting the other warps.  (One warp per SM
+ * sub-partition makes this epilogue bound by its instruction count: with a
+ * TMEM lane per row, 2-byte stores of 32-row pieces took 134 us for an
+ * 8191 x 8191 C at K = 33, a four-warp exchange through shared memory 224.)
+ *
+ * Column j of the 32 sits at pitch 272 bytes, at the same offset within 16
+ * bytes as in C, so that each whole 16-byte chunk of a column moves as one
+ * aligned vector between shared and global memory, two columns per warp
+ * instruction; a column's ends (fewer than 8 rows each) move as 2-byte
+ * elements. */
+constexpr int COLS_ROWS = 128;
+constexpr uint32_t COLS_PITCH = 2 * COLS_ROWS + 16; /* the rows + 16 bytes of alignment */
+constexpr uint32_t COLS_WARP_BYTES = 32 * COLS_PITCH;
+
+/* whole chunks of the 32 columns at C (ldc apart; `rows` <= COLS_ROWS rows,
+ * `cols` valid columns) from shared to global memory (STORE) or back */
+template <bool STORE>
+__device__ __forceinline__ void cols_copy(uint8_t *buf, __half *C, long long ldc, int rows,
+                                          int cols) {
+  const int lane = threadIdx.x & 31;
+  const int c16 = 16 * (lane & 15);
+  const int j0 = lane >> 4;
+  const int bytes = 2 * rows;
+  uint8_t *g = reinterpret_cast<uint8_t *>(C + (long long)j0 * ldc);
+  uint8_t *s = buf + j0 * COLS_PITCH + c16;
+#pragma unroll 1
+  for (int h = 0; h < 32; h += 16) {
+    uint4 v[8];
+    uint8_t *at[8];
+    bool on[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) { /* every load before the first store */
+      const int mis = (int)(reinterpret_cast<uintptr_t>(g) & 15);
+      on[i] = h + 2 * i + j0 < cols && c16 >= mis && c16 + 16 <= mis + bytes;
+      at[i] = g - mis + c16;
+      g += 4 * ldc; /* two columns */
+      if (on[i])
+        v[i] = STORE ? *reinterpret_cast<const uint4 *>(s + 2 * i * COLS_PITCH)
+                     : *reinterpret_cast<const uint4 *>(at[i]);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+      if (on[i]) *reinterpret_cast<uint4 *>(STORE ? at[i] : s + 2 * i * COLS_PITCH) = v[i];
+    s += 16 * COLS_PITCH;
+  }
+}
+
+/* the ends of this lane's column: the rows before its first and after its
+ * last whole chunk */
+template <bool STORE>
+__device__ __forceinline__ void cols_ends(uint8_t *sb, __half *g, int rows) {
+  const int mis = (int)(reinterpret_cast<uintptr_t>(g) & 15);
+  __half *s = reinterpret_cast<__half *>(sb + mis);
+  const int head = mis ? (16 - mis) >> 1 : 0;
+  const int last = (((mis + 2 * rows) & ~15) - mis) >> 1;
+  const int tail = last > head ? last : head;
+#pragma unroll
+  for (int i = 0; i < 7; ++i)
+    if (i < head && i < rows) {
+      if (STORE) g[i] = s[i];
+      else s[i] = g[i];
+    }
+#pragma unroll
+  for (int i = 0; i < 7; ++i)
+    if (tail + i < rows) {
+      if (STORE) g[tail + i] = s[tail + i];
+      else s[tail + i] = g[tail + i];
+    }
+}
+
+/* One warp's 32 columns x `width` rows of C: TMEM lane i (of this warp) is
+ * column i, `width` TMEM columns at tbase are consecutive rows; rows / cols
+ * valid; C the first of them.  C = alpha * acc (+ beta * C). */
+__device__ __forceinline__ void cols_tile(uint8_t *buf, uint32_t tbase, int width, __half *C,
+                                          long long ldc, int rows, int cols, float alpha,
+                                          float beta, bool ld_c) {
+  const int lane = threadIdx.x & 31;
+  uint8_t *sb = buf + lane * COLS_PITCH;
+  if (rows > width) rows = width;
+#pragma unroll 1
+  for (int r0 = 0; r0 < rows; r0 += COLS_ROWS) {
+    const int nr = rows - r0 < COLS_ROWS ? rows - r0 : COLS_ROWS;
+    __half *Cp = C + r0;
+    __half *col = Cp + (long long)lane * ldc;
+    const int mis = (int)(reinterpret_cast<uintptr_t>(col) & 15);
+    uint32_t *w = reinterpret_cast<uint32_t *>(sb + (mis & ~3));
+    const uint32_t sft = (mis & 2) * 8; /* 16 when the column starts in a word's upper half */
+    __syncwarp(); /* the previous rows have been copied out */
+    if (ld_c) {
+      cols_copy<false>(buf, Cp, ldc, nr, cols);
+      if (lane < cols) cols_ends<false>(sb, col, nr);
+      __syncwarp();
+    }
+    uint32_t carry = ld_c ? w[0] : 0u, old = carry;
+#pragma unroll 1
+    for (int g = 0; g < nr; g += 32) {
+      uint32_t r[32];
+      tmem_ld_32x32b_x32(tbase + r0 + g, r);
+      tmem_ld_wait();
+      uint32_t *wg = w + g / 2;
+      if (ld_c) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          /* rows 2i, 2i + 1 of the group: words i and i + 1 of the column */
+          const uint32_t next = wg[i + 1];
+          const uint32_t c2 = __funnelshift_r(old, next, sft);
+          old = next;
+          const __half2 h = *reinterpret_cast<const __half2 *>(&c2);
+          r[2 * i] = __float_as_uint(
+              fmaf(beta, __low2float(h), alpha * __uint_as_float(r[2 * i])));
+          r[2 * i + 1] = __float_as_uint(
+              fmaf(beta, __high2float(h), alpha * __uint_as_float(r[2 * i + 1])));
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          r[i] = __float_as_uint(alpha * __uint_as_float(r[i]));
+      }
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        const __half2 h =
+            __floats2half2_rn(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+        const uint32_t hw = *reinterpret_cast<const uint32_t *>(&h);
+        wg[i] = __funnelshift_l(carry, hw, sft);
+        carry = hw;
+      }
+      /* the last row of a shifted column; the next group rewrites the word */
+      if (!ld_c || g + 32 >= nr) wg[16] = __funnelshift_l(carry, 0u, sft);
+    }
+    __syncwarp();
+    cols_copy<true>(buf, Cp, ldc, nr, cols);
+    if (lane < cols) cols_ends<true>(sb, col, nr);
+  }
+}
 
 }  // namespace tc
 }  // namespace hcbk

@@ -330,6 +330,41 @@ template <typename OutT> struct EpiAlphaBeta {
   }
 };
 
+/* f16 C that TMA cannot address, as the transposed product (m counts C's
+ * columns, n its rows): see cols_tile.  EW = 8 warps share the rows of a TMEM
+ * lane quadrant between two (one warp per scheduler leaves most issue slots
+ * to latency) and take the room of one more pipeline stage; EW = 4 keep it. */
+template <int EW> struct EpiColsH {
+  static constexpr bool INPLACE = false;
+  static constexpr bool PLANE_BATCH = false;
+  static constexpr int EPI_WARPS = EW;
+  static constexpr uint32_t OUT_WARP_BYTES = COLS_WARP_BYTES;
+  static constexpr uint32_t OUT_SMEM = EPI_WARPS * OUT_WARP_BYTES;
+
+  /* beta != 0: while the tile's MMAs run, ask L2 for the lane's rows of its
+   * column */
+  template <int BN>
+  static __device__ __forceinline__ void prefetch_c(const TcParams &p, int m0, int n0,
+                                                    OutStage &) {
+    const int m = m0 + (int)(threadIdx.x & 31);
+    if (!p.beta_nonzero || m >= p.m) return;
+    const __half *C = static_cast<const __half *>(p.c) + n0 + (long long)m * p.ldc;
+    const int rows = p.n - n0 < BN ? p.n - n0 : BN;
+    for (int r = 0; r < rows; r += 64) /* 128-byte lines */
+      asm volatile("prefetch.global.L2 [%0];" ::"l"(C + r));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(C + rows - 1));
+  }
+
+  template <int BN, int NACC>
+  static __device__ __forceinline__ void run(const TcParams &p, uint32_t tbase, int m, int n0,
+                                             OutStage &os) {
+    static_assert(NACC == 1, "one accumulator");
+    const int m0 = m - (int)(threadIdx.x & 31);
+    cols_tile(os.box, tbase, BN, static_cast<__half *>(p.c) + n0 + (long long)m0 * p.ldc, p.ldc,
+              p.n - n0, p.m - m0, p.alpha, p.beta, p.beta_nonzero != 0);
+  }
+};
+
 /* Modular epilogue of the CRT scheme, reducing in place in TMEM.
  * With f16 residues |r| <= 127 (moduli <= 255) the tensor core's f32 sums
  * are exact integers while below 2^24: 1024 * 127^2 + 1.5 * 255 < 2^24.
@@ -479,8 +514,8 @@ struct EpiI32Cat {
  * accumulator. */
 template <class E, class = void> struct CatK : std::false_type {};
 /* epilogue warps (EPI_WARPS, default 4): with 8, two warps share each TMEM
- * lane quadrant and take half of the tile's columns each (plane-batched
- * TMA-store epilogues only) */
+ * lane quadrant and take half of the tile's columns each (tiles whose
+ * accumulator is read once) */
 template <class E, class = void> struct EpiWarps {
   static constexpr int value = 4;
 };
@@ -694,8 +729,8 @@ __global__ void __launch_bounds__(64 + 32 * EpiWarps<EPI>::value, 1)
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tempty + 2);
   uint64_t *obar = tempty + 4; /* output staging: two C-load barriers per epilogue warp */
   constexpr int EW = EpiWarps<EPI>::value;
-  static_assert(EW == 4 || (EW == 8 && EPI::PLANE_BATCH && !EPI::INPLACE && BN % 128 == 0),
-                "eight epilogue warps: plane-batched TMA-store epilogues");
+  static_assert(EW == 4 || (EW == 8 && PROMOTE_KB == 0 && !EPI::INPLACE && BN % 128 == 0),
+                "eight epilogue warps split the columns of a tile that is read once");
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -985,7 +1020,9 @@ __global__ void __launch_bounds__(64 + 32 * EpiWarps<EPI>::value, 1)
       const TileMN tc_ = tile_mn(tt, p.tiles_m, p.tiles_n);
       const int tm = tc_.m, tn = tc_.n;
       const int m = (tm * CG + (int)rank) * BM + q * 32 + lane;
-      if constexpr (Cfg::OUT_BYTES > 0) EPI::template prefetch_c<BN>(p, m - lane, tn * BN, ostage);
+      constexpr int COLS = BN / (EW / 4); /* this warp's columns */
+      if constexpr (Cfg::OUT_BYTES > 0)
+        EPI::template prefetch_c<COLS>(p, m - lane, tn * BN + half * COLS, ostage);
       else if constexpr (EpiL2Prefetch<EPI>::value && !EPI::PLANE_BATCH)
         EPI::template prefetch_c_l2<BN>(p, m, tn * BN);
       if constexpr (PROMOTE_KB == 0) {
@@ -996,12 +1033,12 @@ __global__ void __launch_bounds__(64 + 32 * EpiWarps<EPI>::value, 1)
         tc_fence_after();
         const uint32_t tbase =
             tmem_base + (static_cast<uint32_t>(q * 32) << 16) + b * Cfg::ACC_COLS;
-        if constexpr (EPI::PLANE_BATCH) {
-          constexpr int COLS = BN / (EW / 4); /* this warp's columns */
+        if constexpr (EPI::PLANE_BATCH)
           EPI::template final_store<COLS>(p, tbase + half * COLS, ostage.box, m - lane,
                                           tn * BN + half * COLS, plane);
-        } else
-          EPI::template run<BN, R::NACC>(p, tbase, m, tn * BN, ostage);
+        else
+          EPI::template run<COLS, R::NACC>(p, tbase + half * COLS, m, tn * BN + half * COLS,
+                                           ostage);
         tc_fence_before();
         __syncwarp();
         release(b);
@@ -1204,6 +1241,12 @@ extern "C" int hcbk_encode_out_2d(void *map, void *base, uint64_t rows, uint64_t
                       rows, cols, ld);
 }
 
+template <int BN, int STAGES, int EW, int CG> static int launch_cols(TcParams &p, void *stream) {
+  static_assert(TcCfg<BN, STAGES, RecipeSingle, 0, 2, CG, EpiColsH<EW>::OUT_SMEM>::OUT_BYTES > 0,
+                "the columns' staging fits beside the stages");
+  return launch_tc<BN, STAGES, RecipeSingle, 0, EpiColsH<EW>, 0, 2, CG>(p, stream);
+}
+
 /* f16 operands straight from the caller's matrices (column-major canonical). */
 static int hgemm_tc_impl(const hcbk_gemm_args *a, int bn, int pair, int *err, void *stream,
                          int inject_skip_load) {
@@ -1211,31 +1254,9 @@ static int hgemm_tc_impl(const hcbk_gemm_args *a, int bn, int pair, int *err, vo
       a->op_b == HCBK_OP_C)
     return HCBK_ERR_ARGS;
   if (a->m > 0x7fffffff || a->n > 0x7fffffff || a->k > 0x7fffffff) return HCBK_ERR_ARGS;
+  if ((bn != 128 && bn != 256) || (pair && bn != 256)) return HCBK_ERR_ARGS;
   TcParams p;
   memset(&p, 0, sizeof(p));
-  p.m = (int)a->m;
-  p.n = (int)a->n;
-  p.k = (int)a->k;
-  const __half *A = static_cast<const __half *>(a->a) + a->a_off;
-  const __half *B = static_cast<const __half *>(a->b) + a->b_off;
-  /* op(A) = A: column-major M x K, M contiguous (MN-major);  op(A) = A^T: K contiguous */
-  p.a_mn = (a->op_a == HCBK_OP_N);
-  /* op(B) = B: K x N, K contiguous (K-major);  op(B) = B^T: N contiguous */
-  p.b_mn = (a->op_b != HCBK_OP_N);
-  const auto F16 = CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
-  int rc;
-  if (p.a_mn)
-    rc = make_map(&p.ta[0], F16, 2, A, a->m, a->k, a->lda, 64, 64);
-  else
-    rc = make_map(&p.ta[0], F16, 2, A, a->k, a->m, a->lda, 64, BM);
-  if (rc) return rc;
-  if ((bn != 128 && bn != 256) || (pair && bn != 256)) return HCBK_ERR_ARGS;
-  const uint32_t bn_box = (uint32_t)(pair ? bn / 2 : bn); /* B rows per CTA */
-  if (p.b_mn)
-    rc = make_map(&p.tb[0], F16, 2, B, a->n, a->k, a->ldb, 64, 64);
-  else
-    rc = make_map(&p.tb[0], F16, 2, B, a->k, a->n, a->ldb, 64, bn_box);
-  if (rc) return rc;
   p.c = static_cast<__half *>(a->c) + a->c_off;
   p.ldc = a->ldc;
   p.alpha = (float)a->alpha_re;
@@ -1243,9 +1264,37 @@ static int hgemm_tc_impl(const hcbk_gemm_args *a, int bn, int pair, int *err, vo
   p.beta_nonzero = a->beta_re != 0.0;
   p.err = err;
   /* C tensor-map addressable: the epilogue stages 32 x 32 boxes in shared
-   * memory, reading C (beta != 0) and writing it by TMA */
+   * memory, reading C (beta != 0) and writing it by TMA; else the transposed
+   * product C^T = op(B)^T op(A)^T, whose epilogue holds C by columns */
   p.out_tma =
       make_map_out(&p.tc, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p.c, a->m, a->n, a->ldc) == HCBK_OK;
+  const bool swap = !p.out_tma && !inject_skip_load;
+  p.m = (int)(swap ? a->n : a->m);
+  p.n = (int)(swap ? a->m : a->n);
+  p.k = (int)a->k;
+  /* the kernel's first operand is p.m x K, the second K x p.n; an operand is
+   * MN-major when its non-K dimension is contiguous: op(A) = A (M x K
+   * column-major), op(B) = B^T */
+  const bool a_mn = a->op_a == HCBK_OP_N, b_mn = a->op_b != HCBK_OP_N;
+  p.a_mn = swap ? b_mn : a_mn;
+  p.b_mn = swap ? a_mn : b_mn;
+  const __half *A = static_cast<const __half *>(a->a) + a->a_off;
+  const __half *B = static_cast<const __half *>(a->b) + a->b_off;
+  const __half *P0 = swap ? B : A, *P1 = swap ? A : B;
+  const int64_t ld0 = swap ? a->ldb : a->lda, ld1 = swap ? a->lda : a->ldb;
+  const auto F16 = CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  int rc;
+  if (p.a_mn)
+    rc = make_map(&p.ta[0], F16, 2, P0, p.m, a->k, ld0, 64, 64);
+  else
+    rc = make_map(&p.ta[0], F16, 2, P0, a->k, p.m, ld0, 64, BM);
+  if (rc) return rc;
+  const uint32_t bn_box = (uint32_t)(pair ? bn / 2 : bn); /* second-operand rows per CTA */
+  if (p.b_mn)
+    rc = make_map(&p.tb[0], F16, 2, P1, p.n, a->k, ld1, 64, 64);
+  else
+    rc = make_map(&p.tb[0], F16, 2, P1, a->k, p.n, ld1, 64, bn_box);
+  if (rc) return rc;
   using EH = EpiAlphaBeta<__half>;
   if (inject_skip_load) {
     /* one 128 x 128 tile of one 64-wide K block, beta == 0: the only load
@@ -1253,6 +1302,21 @@ static int hgemm_tc_impl(const hcbk_gemm_args *a, int bn, int pair, int *err, vo
     if (a->m > BM || a->n > 128 || a->k > 64 || p.beta_nonzero || pair || bn != 128)
       return HCBK_ERR_ARGS;
     p.inject_skip_load = 1;
+  }
+  if (swap) {
+    /* fewer stages: the columns' staging takes their place.  Eight epilogue
+     * warps where the epilogue bounds the tile, four where its MMAs do;
+     * measured (B200, CTA pairs): 8191 x 8191 x 33 93 against 130 us,
+     * 8378 x 1133 x 777 beta != 0 50 against 57, beta == 0 41 both,
+     * 4095^3 149 against 140. */
+    if (p.k <= (p.beta_nonzero ? 1024 : 512)) {
+      if (pair) return launch_cols<256, 4, 8, 2>(p, stream);
+      if (bn == 256) return launch_cols<256, 3, 8, 1>(p, stream);
+      return launch_cols<128, 4, 8, 1>(p, stream);
+    }
+    if (pair) return launch_cols<256, 5, 4, 2>(p, stream);
+    if (bn == 256) return launch_cols<256, 3, 4, 1>(p, stream);
+    return launch_cols<128, 5, 4, 1>(p, stream);
   }
   if (pair) return launch_tc<256, 6, RecipeSingle, 0, EH, 0, 2, 2>(p, stream);
   if (bn == 256) return launch_tc<256, 4, RecipeSingle, 0, EH>(p, stream);
