@@ -42,7 +42,72 @@ bool aligned16(const void *p, int64_t off, int esz) {
  * launch. */
 constexpr double REALIGN_MIN_MNK = 268435456.0; /* 2^28 */
 
+/* Plain SGEMM / CGEMM: fma_gemm.cu, except where K is too short to pay for
+ * its longer ramp (an unrolled loop fetched for a handful of slabs, a ring
+ * filled by element copies when both operands are K-contiguous).  Measured on
+ * B200, simt_gemm.cu's kernels against fma_gemm.cu's:
+ *   20^3 6.4 / 8.6 us, 600^2 x 96 8.6 / 12.6, 1000^2 x 128 14.7 / 18.6,
+ *   600^2 x 256 15.9 / 15.1, 300^2 x 128 10.6 / 9.3 (the estimates below);
+ *   4096^2 x 96 72 / 70 NN, 72 / 84 TN, 2000^2 x 128 31 / 31 NN, 31 / 37 TN;
+ *   TN 4096^2 x 512 326 / 334, 4096^3 2535 / 2431;
+ *   NT off 16 bytes (element copies along MN) 4095^2 x 2047 1342 / 1397,
+ *   1501^3 with split K 350 / 164;
+ *   complex 64^3 10.6 / 8.5, 600^2 x 16 6.5 / 7.0, 600^2 x 64 TN 11.9 / 12.7. */
+int simt_f32(HcblasB200State *st, const hcbk_gemm_args *a, void *stream, const char **path) {
+  const bool cplx = a->dtype == HCBK_C;
+  if (a->batch_select) return HCBK_ERR_ARGS;
+  const int64_t tiles = tiles_of(a->m, a->n, 64, 64) * a->batch;
+  const int sms = hcbk_sm_count();
+  hcbk_f32_cfg cfg;
+  double us = 0;
+  int rc = hcbk_gemm_f32_plan(cplx, a->m, a->n, a->k, a->batch, &cfg, &us);
+  if (rc) return rc;
+  const bool k_contig = a->op_a != HCBK_OP_N && a->op_b == HCBK_OP_N;
+  if (cplx) {
+    if (a->k <= (k_contig ? 64 : 32) && tiles <= sms) return HCBK_ERR_ARGS;
+  } else {
+    const bool mn_contig = a->op_a == HCBK_OP_N && a->op_b != HCBK_OP_N;
+    const bool aligned = !((a->lda | a->ldb) & 3) &&
+                         (a->a_array || (aligned16(a->a, a->a_off, 4) &&
+                                         aligned16(a->b, a->b_off, 4) &&
+                                         (a->batch == 1 || !((a->stride_a | a->stride_b) & 3))));
+    if (cfg.split == 1 && (a->k <= 128 || (k_contig && aligned && a->k < 1024) ||
+                           (mn_contig && !aligned)))
+      return HCBK_ERR_ARGS;
+    /* the 4 x 4-per-thread kernel: 5 us + 0.0425 us per k while every tile
+     * has an SM, 0.0713 with two tiles on the busiest SM */
+    if (tiles <= sms && 5.0 + 0.0425 * (double)a->k < us) return HCBK_ERR_ARGS;
+    if (tiles <= 2 * sms && 5.0 + 0.0713 * (double)a->k < us) return HCBK_ERR_ARGS;
+  }
+  if (st->autotune) {
+    /* the two tiles, with the planned split (another split would add up K in
+     * another order); beta == 0: the candidates write C, which the final
+     * launch rewrites, otherwise a scratch matrix of C's shape */
+    const bool zero_beta = a->beta_re == 0.0 && a->beta_im == 0.0;
+    TuneTarget tt(a, stream);
+    if (zero_beta || tt.usable())
+      cfg.tile = tune_choice(st, stream, tune_key("simt", a), 2, [&](int i) {
+        const hcbk_gemm_args *t = zero_beta ? a : tt.args();
+        if (!t) return (int)HCBK_ERR_NOMEM;
+        hcbk_f32_cfg c = cfg;
+        c.tile = i;
+        return hcbk_gemm_f32(t, c, stream);
+      }, cfg.tile);
+  }
+  static const char *names[2][2][4] = {
+      {{"simt.s.128x128", "simt.s.128x128.k2", "simt.s.128x128.k4", "simt.s.128x128.k8"},
+       {"simt.s.64x64", "simt.s.64x64.k2", "simt.s.64x64.k4", "simt.s.64x64.k8"}},
+      {{"simt.c.64x64", "simt.c.64x64.k2", "simt.c.64x64.k4", "simt.c.64x64.k8"},
+       {"simt.c.32x32", "simt.c.32x32.k2", "simt.c.32x32.k4", "simt.c.32x32.k8"}}};
+  *path = names[cplx][cfg.tile][cfg.split >= 8 ? 3 : cfg.split >= 4 ? 2 : cfg.split >= 2 ? 1 : 0];
+  return timed_launch(st, stream, *path, [&] { return hcbk_gemm_f32(a, cfg, stream); });
+}
+
 int simt(HcblasB200State *st, const hcbk_gemm_args *a, void *stream, const char **path) {
+  if (a->dtype == HCBK_S || a->dtype == HCBK_C) {
+    const int rc = simt_f32(st, a, stream, path);
+    if (rc != HCBK_ERR_ARGS) return rc;
+  }
   if (a->dtype == HCBK_D && st->dgemm_dmma) {
     /* native FP64 on the DMMA path (mma.sync .f64) */
     *path = "dmma.d.128x128";

@@ -73,6 +73,17 @@ typedef struct hcbk_simt_cfg {
  * accumulation.  Any op, ld, offset, alignment, batch. */
 int hcbk_gemm_simt(const hcbk_gemm_args *args, hcbk_simt_cfg cfg, void *stream);
 
+/* SGEMM / CGEMM on the FP32 FMA pipe: tile 0 = 128 x 128 floats (four warps),
+ * 1 = 64 x 64 (one warp); split = CTAs of a cluster sharing a tile's K range
+ * (1..8).  Any op, ld, offset, alignment, batch. */
+typedef struct hcbk_f32_cfg {
+  int tile, split;
+} hcbk_f32_cfg;
+int hcbk_gemm_f32(const hcbk_gemm_args *args, hcbk_f32_cfg cfg, void *stream);
+/* the tile and split for a problem; *us (optional): the estimated time */
+int hcbk_gemm_f32_plan(int complex, int64_t m, int64_t n, int64_t k, int64_t batch,
+                       hcbk_f32_cfg *cfg, double *us);
+
 /* Native FP64 GEMM on the FP64 tensor path (mma.sync .f64 m16n8k4, 128 x 128
  * CTA tiles).  Any ld, offset, alignment, batch (strided or pointer arrays,
  * batch_select honoured); HCBK_ERR_ARGS for other dtypes. */

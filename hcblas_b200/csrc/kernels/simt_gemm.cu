@@ -5,9 +5,11 @@
  * (lib/src/blas/{s,d,h,c,z}gemm/*kernels*.cpp: col-major NN/NT/TN/TT with
  * ld/offsets, pointer-array batches), in one templated kernel family:
  *
- *   S   binary32 FMA               (reference: sgemm_NN_kernels.cpp:26-136 ...)
+ *   S   binary32 FMA, short K (fma_gemm.cu takes the rest)
+ *                                  (reference: sgemm_NN_kernels.cpp:26-136 ...)
  *   D   binary64 FMA               (dgemm_*kernels*.cpp)
- *   C   complex binary32, 4 real FMAs per complex MAC (cgemm_array_kernels.cpp)
+ *   C   complex binary32, 4 real FMAs per complex MAC, short K
+ *                                  (cgemm_array_kernels.cpp)
  *   Z   complex binary64           (zgemm_*)
  *   H   binary16 storage, binary32 accumulation (the reference accumulates in
  *       half, hgemm_NN_kernels.cpp:40; this library deliberately does not)
@@ -759,7 +761,7 @@ extern "C" int hcbk_gemm_simt(const hcbk_gemm_args *a, hcbk_simt_cfg cfg, void *
   if (a->m <= 0 || a->n <= 0 || a->k <= 0 || a->batch <= 0) return HCBK_ERR_ARGS;
   const bool small = cfg.variant == 1;
   switch (a->dtype) {
-    case HCBK_S:
+    case HCBK_S: /* short K; the rest runs on fma_gemm.cu */
       return small ? launch_cfg<float, 64, 64, 16, 4, 4>(a, st)
                    : launch_cfg<float, 128, 128, 16, 8, 8, 2>(a, st);
     case HCBK_D:
