@@ -108,16 +108,16 @@ int simt(HcblasB200State *st, const hcbk_gemm_args *a, void *stream, const char 
     const int rc = simt_f32(st, a, stream, path);
     if (rc != HCBK_ERR_ARGS) return rc;
   }
-  if (a->dtype == HCBK_D && st->dgemm_dmma) {
-    /* native FP64 on the DMMA path (mma.sync .f64) */
-    *path = "dmma.d.128x128";
-    int rc = timed_launch(st, stream, *path, [&] { return hcbk_dgemm_dmma(a, stream); });
-    if (rc != HCBK_ERR_ARGS) return rc;
-  }
-  if (a->dtype == HCBK_Z && st->dgemm_dmma) {
-    /* native complex FP64: four real DMMA products per fragment set */
-    *path = "dmma.z.128x64";
-    int rc = timed_launch(st, stream, *path, [&] { return hcbk_zgemm_zmma(a, stream); });
+  if ((a->dtype == HCBK_D || a->dtype == HCBK_Z) && st->dgemm_dmma) {
+    /* native FP64 on the DMMA path (mma.sync .f64); complex as four real DMMA
+     * products per fragment set.  The path names are identifiers callers
+     * compare with; the kernels' tiles are 64 x 64. */
+    const bool z = a->dtype == HCBK_Z;
+    const int split = hcbk_gemm_f64_split(z, a->m, a->n, a->k, a->batch);
+    *path = z ? "dmma.z.128x64" : "dmma.d.128x128";
+    int rc = timed_launch(st, stream, *path, [&] {
+      return z ? hcbk_zgemm_zmma(a, split, stream) : hcbk_dgemm_dmma(a, split, stream);
+    });
     if (rc != HCBK_ERR_ARGS) return rc;
   }
   const int sms = hcbk_sm_count();

@@ -84,15 +84,19 @@ int hcbk_gemm_f32(const hcbk_gemm_args *args, hcbk_f32_cfg cfg, void *stream);
 int hcbk_gemm_f32_plan(int complex, int64_t m, int64_t n, int64_t k, int64_t batch,
                        hcbk_f32_cfg *cfg, double *us);
 
-/* Native FP64 GEMM on the FP64 tensor path (mma.sync .f64 m16n8k4, 128 x 128
- * CTA tiles).  Any ld, offset, alignment, batch (strided or pointer arrays,
- * batch_select honoured); HCBK_ERR_ARGS for other dtypes. */
-int hcbk_dgemm_dmma(const hcbk_gemm_args *args, void *stream);
+/* Native FP64 GEMM on the FP64 tensor path (mma.sync .f64); split = CTAs of a
+ * cluster sharing a tile's K range (1..8).  Any ld, offset, alignment, batch
+ * (strided or pointer arrays); HCBK_ERR_ARGS for other dtypes and selective
+ * batches. */
+int hcbk_dgemm_dmma(const hcbk_gemm_args *args, int split, void *stream);
 
 /* Native complex FP64 GEMM on the same path: Re += Ar Br - Ai Bi,
- * Im += Ar Bi + Ai Br as four real DMMA products (128 x 64 CTA tiles); any
- * op (N, T, C), ld, offset, alignment, batch; HCBK_ERR_ARGS for other dtypes. */
-int hcbk_zgemm_zmma(const hcbk_gemm_args *args, void *stream);
+ * Im += Ar Bi + Ai Br as four real DMMA products; any op (N, T, C), ld,
+ * offset, alignment, batch; HCBK_ERR_ARGS for other dtypes and selective
+ * batches. */
+int hcbk_zgemm_zmma(const hcbk_gemm_args *args, int split, void *stream);
+/* the split for a D (Z) problem */
+int hcbk_gemm_f64_split(int complex, int64_t m, int64_t n, int64_t k, int64_t batch);
 
 /* C := beta * C (beta == 0 writes zeros without reading C): the alpha == 0
  * path.  Any dtype, ld, offset, batch. */
