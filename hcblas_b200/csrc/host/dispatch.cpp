@@ -52,7 +52,8 @@ constexpr double REALIGN_MIN_MNK = 268435456.0; /* 2^28 */
  *   TN 4096^2 x 512 326 / 334, 4096^3 2535 / 2431;
  *   NT off 16 bytes (element copies along MN) 4095^2 x 2047 1342 / 1397,
  *   1501^3 with split K 350 / 164;
- *   complex 64^3 10.6 / 8.5, 600^2 x 16 6.5 / 7.0, 600^2 x 64 TN 11.9 / 12.7. */
+ *   complex 64^3 10.6 / 8.5, 600^2 x 16 6.5 / 7.0, 600^2 x 64 TN 11.9 / 12.7,
+ *   2017 x 1373 x 10 24.6 / 25.1. */
 int simt_f32(HcblasB200State *st, const hcbk_gemm_args *a, void *stream, const char **path) {
   const bool cplx = a->dtype == HCBK_C;
   if (a->batch_select) return HCBK_ERR_ARGS;
@@ -64,7 +65,7 @@ int simt_f32(HcblasB200State *st, const hcbk_gemm_args *a, void *stream, const c
   if (rc) return rc;
   const bool k_contig = a->op_a != HCBK_OP_N && a->op_b == HCBK_OP_N;
   if (cplx) {
-    if (a->k <= (k_contig ? 64 : 32) && tiles <= sms) return HCBK_ERR_ARGS;
+    if (a->k <= 16 || (a->k <= (k_contig ? 64 : 32) && tiles <= sms)) return HCBK_ERR_ARGS;
   } else {
     const bool mn_contig = a->op_a == HCBK_OP_N && a->op_b != HCBK_OP_N;
     const bool aligned = !((a->lda | a->ldb) & 3) &&

@@ -5,19 +5,20 @@
  * single calls.
  *
  * Plan: every problem is canonicalised to column-major (row-major handles
- * swap A and B, as run_gemm does), its tensor maps are encoded, and problems
- * are ordered by decreasing work (tiles x K-slabs) so that the kernel's
- * round-robin tile walk ends on the cheapest tiles.  The table (entries, then
- * the count + 1 tile prefix sums) is written into a pinned staging buffer and
- * copied to the device on the handle's stream.  A follow-up call with a
+ * swap A and B, as run_gemm does), and problems are ordered by decreasing work
+ * (tiles x K-slabs) so that the kernel's round-robin tile walk ends on the
+ * cheapest tiles.  The canonical problems and their tile prefix sums go through
+ * a pinned staging buffer to the device, where a kernel writes the table
+ * (tensor maps, shapes, one descriptor per tile).  A follow-up call with a
  * byte-identical problem array (and the same order and device) reuses the
- * device table as it is: no encoding, no copy.
+ * device table as it is.
  */
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstdio>
 #include <cstring>
+#include <utility>
 #include <vector>
 
 #include "dispatch.h"
@@ -164,54 +165,75 @@ int grouped_hgemm(HcblasB200State *st, void *stream, hcblasOrder order, int coun
     }
     gp.key.clear();
     gp.compact_key.clear();
-    std::vector<hcbk_grouped_entry> ent((size_t)count);
-    std::vector<int> ok_idx;
+    /* the problems TMA can address, in their canonical form; the rest run as
+     * single calls */
+    std::vector<hcbk_grouped_problem> ent((size_t)count);
     std::vector<int> fallback;
-    ok_idx.reserve(count);
+    std::vector<std::pair<int64_t, int>> by_work; /* tensor work of the padded tiles */
+    by_work.reserve((size_t)count);
+    int64_t total = 0, all_work = 0;
+    auto addressable = [](const void *p, int64_t ld, int64_t inner) {
+      return (reinterpret_cast<uintptr_t>(p) & 15) == 0 && (ld & 7) == 0 && ld >= inner;
+    };
     for (int i = 0; i < count; ++i) {
       const Canon c = canonical(probs[i], order);
-      int rc = hcbk_grouped_encode(&ent[i], c.op_a, c.op_b, c.m, c.n, c.k, c.a, c.lda, c.b,
-                                   c.ldb, c.c, c.ldc);
-      if (rc == HCBK_OK && !st->grouped_c_tma) ent[i].c_tma = 0; /* direct stores */
-      if (rc == HCBK_OK) ok_idx.push_back(i);
-      else if (rc == HCBK_ERR_ALIGN || rc == HCBK_ERR_ARGS) fallback.push_back(i);
-      else return rc;
-    }
-    auto work = [&](int i) { /* tensor work of a problem's padded tiles */
-      const hcbk_grouped_entry &e = ent[i];
-      return (int64_t)hcbk_grouped_tiles(&e) * e.bn * ((e.k + 63) / 64);
-    };
-    std::stable_sort(ok_idx.begin(), ok_idx.end(),
-                     [&](int x, int y) { return work(x) > work(y); });
-    const int nt = (int)ok_idx.size();
-    if (nt >= (1 << 24)) return HCBK_ERR_ARGS;
-    int64_t total = 0, all_work = 0;
-    for (int j = 0; j < nt; ++j) {
-      total += (int64_t)hcbk_grouped_tiles(&ent[ok_idx[j]]);
-      all_work += work(ok_idx[j]);
+      const bool a_mn = c.op_a == HCBK_OP_N, b_mn = c.op_b != HCBK_OP_N;
+      if (!addressable(c.a, c.lda, a_mn ? c.m : c.k) ||
+          !addressable(c.b, c.ldb, b_mn ? c.n : c.k)) {
+        fallback.push_back(i);
+        continue;
+      }
+      hcbk_grouped_problem &e = ent[(size_t)i];
+      e.a = c.a;
+      e.b = c.b;
+      e.c = c.c;
+      e.lda = (int32_t)c.lda;
+      e.ldb = (int32_t)c.ldb;
+      e.ldc = (int32_t)c.ldc;
+      e.m = (int32_t)c.m;
+      e.n = (int32_t)c.n;
+      e.k = (int32_t)c.k;
+      const int bn = c.n <= 64 ? 64 : 128;
+      e.flags = (bn == 64 ? HCBK_GT_BN64 : 0) | (a_mn ? HCBK_GT_AMN : 0) |
+                (b_mn ? HCBK_GT_BMN : 0);
+      if (st->grouped_c_tma && addressable(c.c, c.ldc, c.m) && (c.m & 7) == 0)
+        e.flags |= HCBK_GT_CTMA; /* as hcbk_encode_out_2d */
+      const int64_t tiles = ((c.m + 127) / 128) * ((c.n + bn - 1) / bn);
+      const int64_t work = tiles * bn * ((c.k + 63) / 64);
+      total += tiles;
+      all_work += work;
       if (total > 0x7fffffff) return HCBK_ERR_ARGS;
+      by_work.emplace_back(-work, i);
     }
-    /* table: entries | tile prefix sums | per-tile descriptors */
+    std::sort(by_work.begin(), by_work.end()); /* largest first, ties in order */
+    const int nt = (int)by_work.size();
+    if (nt >= (1 << 24)) return HCBK_ERR_ARGS;
+    /* device table: entries | problems | tile prefix sums | per-tile
+     * descriptors; the host uploads the problems and the prefix sums, a kernel
+     * builds the rest */
     const size_t ent_bytes = sizeof(hcbk_grouped_entry) * (size_t)nt;
-    const size_t ts_off = (ent_bytes + 255) & ~size_t(255);
-    const size_t td_off = (ts_off + sizeof(int32_t) * ((size_t)nt + 1) + 255) & ~size_t(255);
+    const size_t up_off = (ent_bytes + 255) & ~size_t(255);
+    const size_t prob_bytes = sizeof(hcbk_grouped_problem) * (size_t)nt;
+    const size_t up_bytes = prob_bytes + sizeof(int32_t) * ((size_t)nt + 1);
+    const size_t ts_off = up_off + prob_bytes;
+    const size_t td_off = (up_off + up_bytes + 255) & ~size_t(255);
     const size_t bytes = td_off + 4 * sizeof(int32_t) * (size_t)total;
     total = 0;
     if (nt > 0) {
-      if (!ensure_table(gp, bytes, stream) || !ensure_staging(gp, bytes)) return HCBK_ERR_NOMEM;
+      if (!ensure_table(gp, bytes, stream) || !ensure_staging(gp, up_bytes)) return HCBK_ERR_NOMEM;
+      char *tb = static_cast<char *>(gp.table);
       unsigned char *stg = static_cast<unsigned char *>(gp.staging);
-      auto *dst = reinterpret_cast<hcbk_grouped_entry *>(stg);
-      auto *ts = reinterpret_cast<int32_t *>(stg + ts_off);
-      auto *td = reinterpret_cast<int32_t *>(stg + td_off);
+      auto *dst = reinterpret_cast<hcbk_grouped_problem *>(stg);
+      auto *ts = reinterpret_cast<int32_t *>(stg + prob_bytes);
       for (int j = 0; j < nt; ++j) {
-        const hcbk_grouped_entry &e = ent[ok_idx[j]];
-        std::memcpy(&dst[j], &e, sizeof(e));
+        const hcbk_grouped_problem &e = ent[(size_t)by_work[(size_t)j].second];
+        dst[j] = e;
         ts[j] = (int32_t)total;
-        hcbk_grouped_fill_tiles(&e, j, td + 4 * total);
-        total += (int64_t)hcbk_grouped_tiles(&e);
+        const int bn = e.flags & HCBK_GT_BN64 ? 64 : 128;
+        total += (int64_t)((e.m + 127) / 128) * ((e.n + bn - 1) / bn);
       }
       ts[nt] = (int32_t)total;
-      if (cudaMemcpyAsync(gp.table, stg, bytes, cudaMemcpyHostToDevice,
+      if (cudaMemcpyAsync(tb + up_off, stg, up_bytes, cudaMemcpyHostToDevice,
                           static_cast<cudaStream_t>(stream)) != cudaSuccess)
         return HCBK_ERR_LAUNCH;
       if (!gp.upload_done &&
@@ -223,6 +245,13 @@ int grouped_hgemm(HcblasB200State *st, void *stream, hcblasOrder order, int coun
         cudaEventRecord(static_cast<cudaEvent_t>(gp.upload_done),
                         static_cast<cudaStream_t>(stream));
       }
+      const int rc = timed_launch(st, stream, "tc.h.grouped.table", [&] {
+        return hcbk_grouped_build(reinterpret_cast<const hcbk_grouped_problem *>(tb + up_off),
+                                  reinterpret_cast<const int32_t *>(tb + ts_off),
+                                  reinterpret_cast<hcbk_grouped_entry *>(tb),
+                                  reinterpret_cast<int32_t *>(tb + td_off), nt, stream);
+      });
+      if (rc) return rc;
     }
     gp.count = nt;
     gp.total_tiles = (int)total;
@@ -246,7 +275,7 @@ int grouped_hgemm(HcblasB200State *st, void *stream, hcblasOrder order, int coun
     g.total_tiles = gp.total_tiles;
     g.alpha = alpha;
     g.beta = beta;
-    g.device_maps = 0;
+    g.device_maps = 1;
     g.tile_desc =
         reinterpret_cast<const int32_t *>(static_cast<char *>(gp.table) + gp.tile_desc_offset);
     g.uniform_tiles = 0;

@@ -529,10 +529,12 @@ int hcbk_grouped_encode(hcbk_grouped_entry *e, int op_a, int op_b, int64_t m, in
  * HCBK_ERR_ALIGN when TMA cannot address C. */
 int hcbk_encode_out_2d(void *map, void *base, uint64_t rows, uint64_t cols, uint64_t ld);
 
-/* tiles of an encoded problem: tiles_m * ceil(n / bn) */
+/* tiles of an encoded problem: tiles_m * ceil(n / bn); its HCBK_GT_* flags */
 int hcbk_grouped_tiles(const hcbk_grouped_entry *e);
 
-/* Per-tile descriptors of the grouped kernels (host tables): four int32 per
+int hcbk_grouped_tile_flags(const hcbk_grouped_entry *e);
+
+/* Per-tile descriptors of the grouped kernels: four int32 per
  * tile {problem | flags << 24, tile row, tile column, k}; problem < 2^24. */
 enum {
   HCBK_GT_BN64 = 1, /* 64-wide tiles */
@@ -541,9 +543,26 @@ enum {
   HCBK_GT_CTMA = 8, /* C through tensor stores */
   HCBK_GT_SKIP = 16 /* not computed by the grouped kernel */
 };
-int hcbk_grouped_tile_flags(const hcbk_grouped_entry *e);
 /* the descriptors of every tile of problem `problem` (entry e) into desc */
 void hcbk_grouped_fill_tiles(const hcbk_grouped_entry *e, int problem, int32_t *desc);
+
+/* One problem as the host hands it to the table builder: column-major f16
+ * C(m x n) = op(A) op(B) with TMA-addressable A and B; flags HCBK_GT_* (64-wide
+ * tiles exactly when n <= 64, C through tensor stores only where
+ * hcbk_encode_out_2d would take it). */
+typedef struct alignas(16) hcbk_grouped_problem {
+  const void *a;
+  const void *b;
+  void *c;
+  int32_t lda, ldb, ldc;
+  int32_t m, n, k;
+  int32_t flags;
+} hcbk_grouped_problem;
+/* The grouped HGEMM's table on the device: entries of every problem (tensor
+ * maps written by tensormap.replace, the words hcbk_grouped_encode would give)
+ * and the descriptors of their tiles, problem i's from tile_start[i] on. */
+int hcbk_grouped_build(const hcbk_grouped_problem *problems, const int32_t *tile_start,
+                       hcbk_grouped_entry *table, int32_t *tile_desc, int count, void *stream);
 
 /* Device-side table of a uniform pointer-array batch: entry i is *tmpl with
  * the addresses of its maps replaced by a_arr[i] + a_off_bytes +

@@ -253,6 +253,21 @@ __device__ __forceinline__ void tensormap_replace_address(void *map, const void 
                : "memory");
 }
 
+/* dimension ORD's extent, and the byte stride of dimension ORD + 1 */
+template <int ORD> __device__ __forceinline__ void tensormap_replace_dim(void *map, uint32_t n) {
+  asm volatile("tensormap.replace.tile.global_dim.global.b1024.b32 [%0], %2, %1;" ::"l"(
+                   reinterpret_cast<uint64_t>(map)),
+               "r"(n), "n"(ORD)
+               : "memory");
+}
+template <int ORD>
+__device__ __forceinline__ void tensormap_replace_stride(void *map, uint64_t bytes) {
+  asm volatile("tensormap.replace.tile.global_stride.global.b1024.b64 [%0], %2, %1;" ::"l"(
+                   reinterpret_cast<uint64_t>(map)),
+               "l"(bytes), "n"(ORD)
+               : "memory");
+}
+
 __device__ __forceinline__ void tensormap_release() {
   asm volatile("fence.proxy.tensormap::generic.release.gpu;" ::: "memory");
 }
