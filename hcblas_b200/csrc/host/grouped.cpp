@@ -220,11 +220,17 @@ int grouped_hgemm(HcblasB200State *st, void *stream, hcblasOrder order, int coun
     const size_t bytes = td_off + 4 * sizeof(int32_t) * (size_t)total;
     total = 0;
     if (nt > 0) {
-      if (!ensure_table(gp, bytes, stream) || !ensure_staging(gp, up_bytes)) return HCBK_ERR_NOMEM;
+      /* a few problems go to the builder as its parameters, more through the
+       * staging buffer */
+      const bool inlined = nt <= HCBK_GROUPED_INLINE;
+      if (!ensure_table(gp, bytes, stream) || (!inlined && !ensure_staging(gp, up_bytes)))
+        return HCBK_ERR_NOMEM;
       char *tb = static_cast<char *>(gp.table);
+      hcbk_grouped_problem few[HCBK_GROUPED_INLINE];
+      int32_t few_ts[HCBK_GROUPED_INLINE + 1];
       unsigned char *stg = static_cast<unsigned char *>(gp.staging);
-      auto *dst = reinterpret_cast<hcbk_grouped_problem *>(stg);
-      auto *ts = reinterpret_cast<int32_t *>(stg + prob_bytes);
+      hcbk_grouped_problem *dst = inlined ? few : reinterpret_cast<hcbk_grouped_problem *>(stg);
+      int32_t *ts = inlined ? few_ts : reinterpret_cast<int32_t *>(stg + prob_bytes);
       for (int j = 0; j < nt; ++j) {
         const hcbk_grouped_problem &e = ent[(size_t)by_work[(size_t)j].second];
         dst[j] = e;
@@ -233,23 +239,26 @@ int grouped_hgemm(HcblasB200State *st, void *stream, hcblasOrder order, int coun
         total += (int64_t)((e.m + 127) / 128) * ((e.n + bn - 1) / bn);
       }
       ts[nt] = (int32_t)total;
-      if (cudaMemcpyAsync(tb + up_off, stg, up_bytes, cudaMemcpyHostToDevice,
-                          static_cast<cudaStream_t>(stream)) != cudaSuccess)
-        return HCBK_ERR_LAUNCH;
-      if (!gp.upload_done &&
-          cudaEventCreateWithFlags(reinterpret_cast<cudaEvent_t *>(&gp.upload_done),
-                                   cudaEventDisableTiming) != cudaSuccess) {
-        gp.upload_done = nullptr;
-        cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
-      } else {
-        cudaEventRecord(static_cast<cudaEvent_t>(gp.upload_done),
-                        static_cast<cudaStream_t>(stream));
+      if (!inlined) {
+        if (cudaMemcpyAsync(tb + up_off, stg, up_bytes, cudaMemcpyHostToDevice,
+                            static_cast<cudaStream_t>(stream)) != cudaSuccess)
+          return HCBK_ERR_LAUNCH;
+        if (!gp.upload_done &&
+            cudaEventCreateWithFlags(reinterpret_cast<cudaEvent_t *>(&gp.upload_done),
+                                     cudaEventDisableTiming) != cudaSuccess) {
+          gp.upload_done = nullptr;
+          cudaStreamSynchronize(static_cast<cudaStream_t>(stream));
+        } else {
+          cudaEventRecord(static_cast<cudaEvent_t>(gp.upload_done),
+                          static_cast<cudaStream_t>(stream));
+        }
+        dst = reinterpret_cast<hcbk_grouped_problem *>(tb + up_off);
+        ts = reinterpret_cast<int32_t *>(tb + ts_off);
       }
       const int rc = timed_launch(st, stream, "tc.h.grouped.table", [&] {
-        return hcbk_grouped_build(reinterpret_cast<const hcbk_grouped_problem *>(tb + up_off),
-                                  reinterpret_cast<const int32_t *>(tb + ts_off),
-                                  reinterpret_cast<hcbk_grouped_entry *>(tb),
-                                  reinterpret_cast<int32_t *>(tb + td_off), nt, stream);
+        return hcbk_grouped_build(dst, ts, reinterpret_cast<hcbk_grouped_entry *>(tb),
+                                  reinterpret_cast<int32_t *>(tb + td_off), nt, inlined ? 1 : 0,
+                                  stream);
       });
       if (rc) return rc;
     }

@@ -27,6 +27,8 @@
 #include <stdint.h>
 #include <string.h>
 
+#include <type_traits>
+
 #include "hcbk.h"
 #include "split_bf16.cuh"
 #include "tc_common.cuh"
@@ -467,12 +469,28 @@ struct BuildArgs {
   int count;
 };
 constexpr int64_t TMPL_SPAN = 128 << 10;
+/* a few problems travel as kernel parameters instead of through a copy */
+struct BuildInline {
+  hcbk_grouped_problem problems[HCBK_GROUPED_INLINE];
+  int32_t tile_start[HCBK_GROUPED_INLINE];
+};
+struct BuildNone {};
 
-__global__ void __launch_bounds__(128) grouped_build_kernel(const __grid_constant__ BuildArgs a) {
+template <class Inline>
+__global__ void __launch_bounds__(128)
+grouped_build_kernel(const __grid_constant__ BuildArgs a, const __grid_constant__ Inline in) {
   const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   if (i >= a.count) return;
-  const hcbk_grouped_problem p = a.problems[i];
+  hcbk_grouped_problem p;
+  int first;
+  if constexpr (std::is_same<Inline, BuildInline>::value) {
+    p = in.problems[i];
+    first = in.tile_start[i];
+  } else {
+    p = a.problems[i];
+    first = a.tile_start[i];
+  }
   hcbk_grouped_entry *e = a.table + i;
   const int a_mn = p.flags & HCBK_GT_AMN ? 1 : 0, b_mn = p.flags & HCBK_GT_BMN ? 1 : 0;
   const int bn = p.flags & HCBK_GT_BN64 ? 64 : 128;
@@ -511,7 +529,7 @@ __global__ void __launch_bounds__(128) grouped_build_kernel(const __grid_constan
     e->skip = 0;
   }
   const int tiles_m = (p.m + BM - 1) / BM, tiles = tiles_m * ((p.n + bn - 1) / bn);
-  int4 *d = a.tile_desc + a.tile_start[i];
+  int4 *d = a.tile_desc + first;
   for (int t = lane; t < tiles; t += 32)
     d[t] = make_int4((int)((unsigned)i | ((unsigned)p.flags << 24)), t % tiles_m, t / tiles_m, p.k);
 }
@@ -973,7 +991,7 @@ extern "C" int hcbk_grouped_ptr_table(const hcbk_grouped_entry *tmpl, hcbk_group
 
 extern "C" int hcbk_grouped_build(const hcbk_grouped_problem *problems, const int32_t *tile_start,
                                   hcbk_grouped_entry *table, int32_t *tile_desc, int count,
-                                  void *stream) {
+                                  int on_host, void *stream) {
   using namespace hcbk::grouped;
   if (count <= 0 || count >= (1 << 24) || (reinterpret_cast<uintptr_t>(table) & 127) ||
       (reinterpret_cast<uintptr_t>(tile_desc) & 15))
@@ -993,7 +1011,17 @@ extern "C" int hcbk_grouped_build(const hcbk_grouped_problem *problems, const in
   a.table = table;
   a.tile_desc = reinterpret_cast<int4 *>(tile_desc);
   a.count = count;
-  grouped_build_kernel<<<(unsigned)((count + 3) / 4), 128, 0, static_cast<cudaStream_t>(stream)>>>(a);
+  const unsigned blocks = (unsigned)((count + 3) / 4);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  if (on_host) {
+    if (count > HCBK_GROUPED_INLINE) return HCBK_ERR_ARGS;
+    BuildInline in;
+    memcpy(in.problems, problems, sizeof(hcbk_grouped_problem) * (size_t)count);
+    memcpy(in.tile_start, tile_start, sizeof(int32_t) * (size_t)count);
+    grouped_build_kernel<<<blocks, 128, 0, st>>>(a, in);
+  } else {
+    grouped_build_kernel<<<blocks, 128, 0, st>>>(a, BuildNone());
+  }
   return cudaGetLastError() == cudaSuccess ? HCBK_OK : HCBK_ERR_LAUNCH;
 }
 

@@ -560,9 +560,13 @@ typedef struct alignas(16) hcbk_grouped_problem {
 } hcbk_grouped_problem;
 /* The grouped HGEMM's table on the device: entries of every problem (tensor
  * maps written by tensormap.replace, the words hcbk_grouped_encode would give)
- * and the descriptors of their tiles, problem i's from tile_start[i] on. */
+ * and the descriptors of their tiles, problem i's from tile_start[i] on.
+ * problems and tile_start are device memory or, on_host != 0 and count <=
+ * HCBK_GROUPED_INLINE, host memory (handed over as kernel parameters). */
+#define HCBK_GROUPED_INLINE 256
 int hcbk_grouped_build(const hcbk_grouped_problem *problems, const int32_t *tile_start,
-                       hcbk_grouped_entry *table, int32_t *tile_desc, int count, void *stream);
+                       hcbk_grouped_entry *table, int32_t *tile_desc, int count, int on_host,
+                       void *stream);
 
 /* Device-side table of a uniform pointer-array batch: entry i is *tmpl with
  * the addresses of its maps replaced by a_arr[i] + a_off_bytes +

@@ -27,7 +27,7 @@ def test_build_matches_encode(handle):
     i64, vp = ctypes.c_int64, ctypes.c_void_p
     L.hcbk_grouped_encode.argtypes = [vp, ctypes.c_int, ctypes.c_int, i64, i64, i64, vp, i64, vp,
                                       i64, vp, i64]
-    L.hcbk_grouped_build.argtypes = [vp, vp, vp, vp, ctypes.c_int, vp]
+    L.hcbk_grouped_build.argtypes = [vp, vp, vp, vp, ctypes.c_int, ctypes.c_int, vp]
     pool = hb.DeviceArray(handle, nbytes=1 << 20, dtype=np.uint8)  # addresses only
     rng = np.random.default_rng(0)
     sizes = [1, 7, 8, 16, 63, 64, 65, 127, 128, 129, 255, 256, 257, 511, 512, 1000, 1024, 2048]
@@ -56,15 +56,18 @@ def test_build_matches_encode(handle):
         tm, tn = -(-m // 128), -(-n // bn)
         descs += [(i | flags << 24, t % tm, t // tm, k) for t in range(tm * tn)]
         ts.append(ts[-1] + tm * tn)
-    dp = hb.DeviceArray(handle, np.array(probs, PROBLEM).view(np.uint8))
-    dts = hb.DeviceArray(handle, np.array(ts, np.int32))
-    table = hb.DeviceArray(handle, np.zeros(ENTRY * len(probs), np.uint8))
-    td = hb.DeviceArray(handle, np.full(4 * ts[-1] + 4, -1, np.int32))
-    assert L.hcbk_grouped_build(dp.ptr, dts.ptr, table.ptr, td.ptr, len(probs), None) == 0
-    got = table.download().reshape(-1, ENTRY)
-    for i, w in enumerate(want):
-        assert np.array_equal(got[i, :MAPS], w[:MAPS]), (i, probs[i])
-        assert np.array_equal(got[i, MAPS:MAPS + 52], w[MAPS:MAPS + 52]), (i, probs[i])
-    d = td.download()
-    assert np.array_equal(d[:-4].reshape(-1, 4), np.array(descs, np.int64).astype(np.int32))
-    assert (d[-4:] == -1).all()
+    hp, hts = np.array(probs, PROBLEM), np.array(ts, np.int32)
+    dp, dts = hb.DeviceArray(handle, hp.view(np.uint8)), hb.DeviceArray(handle, hts)
+    for count, on_host in ((len(probs), 0), (256, 1), (1, 1)):  # copied, handed over as parameters
+        tiles = ts[count]
+        table = hb.DeviceArray(handle, np.zeros(ENTRY * count, np.uint8))
+        td = hb.DeviceArray(handle, np.full(4 * tiles + 4, -1, np.int32))
+        src = (hp.ctypes.data, hts.ctypes.data) if on_host else (dp.ptr, dts.ptr)
+        assert L.hcbk_grouped_build(*src, table.ptr, td.ptr, count, on_host, None) == 0
+        got = table.download().reshape(-1, ENTRY)
+        for i, w in enumerate(want[:count]):
+            assert np.array_equal(got[i, :MAPS], w[:MAPS]), (i, probs[i])
+            assert np.array_equal(got[i, MAPS:MAPS + 52], w[MAPS:MAPS + 52]), (i, probs[i])
+        d = td.download()
+        assert np.array_equal(d[:-4].reshape(-1, 4), np.array(descs[:tiles], np.int64).astype(np.int32))
+        assert (d[-4:] == -1).all()
