@@ -59,6 +59,8 @@ int simt_f32(HcblasB200State *st, const hcbk_gemm_args *a, void *stream, const c
   if (a->batch_select) return HCBK_ERR_ARGS;
   const int64_t tiles = tiles_of(a->m, a->n, 64, 64) * a->batch;
   const int sms = hcbk_sm_count();
+  /* the shortest calls, decided without the estimate (which is at least 7 us) */
+  if (!cplx && tiles <= sms && a->k <= 47) return HCBK_ERR_ARGS;
   hcbk_f32_cfg cfg;
   double us = 0;
   int rc = hcbk_gemm_f32_plan(cplx, a->m, a->n, a->k, a->batch, &cfg, &us);
