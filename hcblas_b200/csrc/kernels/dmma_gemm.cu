@@ -806,6 +806,7 @@ extern "C" int hcbk_gemm_f64_split(int complex, int64_t m, int64_t n, int64_t k,
     const int64_t rem = ctas - full * sms * res, last = (rem + sms - 1) / sms;
     double t = (double)(full * res) * (work / eff[z][res - 1] + extra);
     if (last) t += (double)last * (work / eff[z][last - 1] + extra);
+    if (split > 1) t += 3000; /* the cluster's launch and barriers (60 x 9 x 20: 10.3 -> 12.3 us) */
     if (best == 0 || t < best) {
       best = t;
       choice = split;
