@@ -629,18 +629,23 @@ extern "C" int hcbk_gemm_f32(const hcbk_gemm_args *a, hcbk_f32_cfg cfg, void *st
 }
 
 /* Tile and split from an estimate of the busiest SM's cycles: the slabs of
- * its CTAs at the rate that many resident warps reach, plus each CTA's
- * prologue and epilogue (dearer when a cluster adds up its tile).  The rates
- * and costs were fitted to measured times of every (tile, split) on 16 shapes
- * from 64 x 512 x 100 to 777 x 1133 x 14522; the choice is within 3 % of
- * the fastest on average, 12 % at worst (2048^3).  Splits that are not powers
- * of two pack badly into the GPCs and were never much better. */
+ * its CTAs at the rate that many resident CTAs reach, plus each CTA's prologue
+ * and epilogue (dearer when a cluster adds up its tile, dearest when clusters
+ * queue for more than one wave).  Rates and costs were fitted to measured
+ * times of every (tile, split) on 26 shapes each of SGEMM (256^2 x 4000 to
+ * 2048^3) and CGEMM; the choice is within 1.8 % of the fastest on average,
+ * 18 % at worst.  Splits that are not powers of two pack badly into the GPCs
+ * and were never much better. */
 extern "C" int hcbk_gemm_f32_plan(int complex, int64_t m, int64_t n, int64_t k, int64_t batch,
                                   hcbk_f32_cfg *cfg, double *us) {
-  static const double eff[2][8] = {{.65, .76}, {.31, .49, .54, .57, .60, .62, .62, .63}};
+  static const double eff[3][8] = {
+      {.72, .83},                                /* 128 x 128, real */
+      {.56, .82},                                /* complex */
+      {.33, .52, .54, .62, .62, .62, .62, .70}}; /* 64 x 64 */
   static const int resident[2] = {2, 8};
   static const double slab[2] = {2048, 512}; /* FMA cycles of a slab */
-  static const double cta[2][2] = {{1000, 14000}, {300, 1000}}; /* whole K, split */
+  /* per CTA: whole K, split in one wave, split in several */
+  static const double cta[2][3] = {{1200, 4800, 20000}, {300, 640, 1100}};
   const int sms = hcbk_sm_count();
   const int64_t slabs = (k + BK - 1) / BK;
   double best = 0;
@@ -650,14 +655,15 @@ extern "C" int hcbk_gemm_f32_plan(int complex, int64_t m, int64_t n, int64_t k, 
     const int64_t b = (tile == 0 ? 128 : 64) / (complex ? 2 : 1);
     const int64_t tiles = ((m + b - 1) / b) * ((n + b - 1) / b) * batch;
     const int res = resident[tile];
+    const double *rate = eff[tile ? 2 : complex ? 1 : 0];
     for (int split = 1; split <= MAX_SPLIT && split <= slabs; split *= 2) {
       const double work = (double)((slabs + split - 1) / split) * slab[tile];
-      const double extra = cta[tile][split > 1];
       const int64_t ctas = tiles * split, full = ctas / ((int64_t)sms * res);
       const int64_t rem = ctas - full * sms * res, last = (rem + sms - 1) / sms;
-      double t = (double)(full * res) * (work / eff[tile][res - 1] + extra);
-      if (last) t += (double)last * (work / eff[tile][last - 1] + extra);
-      if (split > 1) t += 1500;
+      const double extra = cta[tile][split == 1 ? 0 : ctas <= (int64_t)sms * res ? 1 : 2];
+      double t = (double)(full * res) * (work / rate[res - 1] + extra);
+      if (last) t += (double)last * (work / rate[last - 1] + extra);
+      if (split > 1) t += 4400;
       if (best == 0 || t < best) {
         best = t;
         cfg->tile = tile;
