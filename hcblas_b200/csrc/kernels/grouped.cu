@@ -174,6 +174,8 @@ __global__ void __launch_bounds__(192, MINB) grouped_hgemm_kernel(const __grid_c
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_wait(); /* the table */
+  grid_launch_dependents();
 
   if (warp == 0) {
     /* ------------------------------------------------ TMA producer -- */
@@ -422,6 +424,7 @@ __global__ void __launch_bounds__(128) grouped_ptr_table_kernel(const __grid_con
    * patches the addresses */
   const int i = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
+  grid_launch_dependents();
   if (i > a.count) return;
   if (lane == 0) a.tile_start[i] = i * a.tiles;
   if (i == a.count) return;
@@ -481,6 +484,7 @@ __global__ void __launch_bounds__(128)
 grouped_build_kernel(const __grid_constant__ BuildArgs a, const __grid_constant__ Inline in) {
   const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
+  grid_launch_dependents();
   if (i >= a.count) return;
   hcbk_grouped_problem p;
   int first;
@@ -1057,8 +1061,20 @@ int launch_grouped_h(const hcbk_grouped_args *g, int *err, void *stream) {
   p.err = err;
   int grid = hcbk_sm_count() * MINB;
   if (g->total_tiles < grid) grid = g->total_tiles;
-  kern<<<grid, 192, Cfg::SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(p);
-  return cudaGetLastError() == cudaSuccess ? HCBK_OK : HCBK_ERR_LAUNCH;
+  cudaLaunchAttribute attr = pdl_attribute(); /* behind the table builder */
+  cudaLaunchConfig_t cfg;
+  memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3((unsigned)grid, 1, 1);
+  cfg.blockDim = dim3(192, 1, 1);
+  cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
+  cfg.stream = static_cast<cudaStream_t>(stream);
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kern, p) != cudaSuccess) {
+    cudaGetLastError();
+    return HCBK_ERR_LAUNCH;
+  }
+  return HCBK_OK;
 }
 }  // namespace
 

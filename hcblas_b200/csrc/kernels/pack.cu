@@ -41,6 +41,7 @@ struct PackPair {
 };
 
 __global__ void pack_kcontig(const __grid_constant__ PackPair pp) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); /* the GEMM waits for its end */
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < pp.total;
        i += (int64_t)gridDim.x * blockDim.x) {
     const int which = i >= pp.units0 ? 1 : 0;
@@ -237,6 +238,7 @@ __device__ __forceinline__ uint4 load8_f16(const uint16_t *s, int valid) {
 }
 
 __global__ void __launch_bounds__(256) realign_f16_kernel(const __grid_constant__ RealignArgs a) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); /* the GEMM waits for its end */
   const int lane = threadIdx.x & 31;
   const int64_t warps = (int64_t)gridDim.x * (blockDim.x >> 5);
   const int64_t total = a.units[0] + a.units[1];

@@ -597,6 +597,9 @@ simt_gemm_kernel(SimtParams<T, typename AccOf<T>::type> p) {
   const int64_t n0 = tile_n * BN;
 
   if (p.sel) {
+    /* launched with the programmatic-serialization attribute: nothing is read
+     * before the kernel ahead (which fills in the flags' other entries) is done */
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     /* a selective pass (usually with nothing selected): the block's threads
      * read its entries' flags together and the block leaves when none is set */
     int any = 0;
@@ -698,6 +701,26 @@ template <class K> static int resident_blocks(K kern, int threads) {
   return per_sm > 0 ? per_sm : 1;
 }
 
+/* launch overlapped with the end of the kernel ahead (selective passes, whose
+ * blocks wait for it before they read anything) */
+template <class K, class P>
+static int launch_after(K kern, dim3 grid, dim3 block, const P &p, cudaStream_t st) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = st;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, kern, p) != cudaSuccess) {
+    cudaGetLastError();
+    return HCBK_ERR_LAUNCH;
+  }
+  return HCBK_OK;
+}
+
 /* MINB: CTAs per SM the register allocation must allow (2 for the FP32
  * tiles: sixteen warps per SM hide the global-load latency of each K-slab
  * better than eight; 64 x 64 tiles, 900 x 900 x 90 NT 19.0 -> 12.8 us) */
@@ -740,6 +763,7 @@ int launch_cfg(const hcbk_gemm_args *a, cudaStream_t st) {
       static const int resident = resident_blocks(kern, (int)block.x);           \
       per_sm = resident;                                                          \
     }                                                                             \
+    if (a->batch_select) return launch_after(kern, grid_of(per_sm), block, p, st); \
     kern<<<grid_of(per_sm), block, 0, st>>>(p);                                   \
     return cudaGetLastError() == cudaSuccess ? HCBK_OK : HCBK_ERR_LAUNCH;         \
   }

@@ -127,6 +127,29 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, int *e
   }
 }
 
+/* --------------------------------------- programmatic dependent launch -- */
+
+/* A kernel launched with the programmatic-serialization attribute may start
+ * while the kernel before it in the stream still runs; all its threads wait
+ * here, before the first access to global memory, until that kernel is done
+ * and its writes are visible (at once when launched the ordinary way).  What
+ * overlaps is the launch itself and the prologue (barriers, TMEM). */
+__device__ __forceinline__ void grid_dependency_wait() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+/* the launch attribute of such a kernel */
+inline cudaLaunchAttribute pdl_attribute() {
+  cudaLaunchAttribute a;
+  a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  a.val.programmaticStreamSerializationAllowed = 1;
+  return a;
+}
+/* in the kernel before: the next one may be scheduled once every block has
+ * passed here (or ended) */
+__device__ __forceinline__ void grid_launch_dependents() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 /* ------------------------------------------------- CTA pair (cluster) -- */
 
 __device__ __forceinline__ uint32_t cluster_ctarank() {

@@ -773,6 +773,7 @@ __global__ void __launch_bounds__(64 + 32 * EpiWarps<EPI>::value, 1)
     __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_dependency_wait(); /* the operands, when a kernel before prepares them */
 
   /* persistent loop over output tiles of (BM * CG) x BN, one per CTA group
    * (times the batched planes of a plane-batched epilogue) */
@@ -1157,16 +1158,17 @@ static int launch_tc(TcParams &p, void *stream) {
   if (dev < 0 || dev >= 64) return HCBK_ERR_LAUNCH;
   cudaLaunchConfig_t cfg;
   memset(&cfg, 0, sizeof(cfg));
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = CG;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute attr[2];
+  attr[0] = pdl_attribute();
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = CG;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
   cfg.blockDim = dim3(64 + 32 * EpiWarps<EPI>::value, 1, 1);
   cfg.dynamicSmemBytes = Cfg::SMEM_BYTES;
   cfg.stream = static_cast<cudaStream_t>(stream);
   cfg.attrs = attr;
-  cfg.numAttrs = CG == 2 ? 1 : 0;
+  cfg.numAttrs = CG == 2 ? 2 : 1;
   if (!attr_set[dev]) {
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              Cfg::SMEM_BYTES) != cudaSuccess)

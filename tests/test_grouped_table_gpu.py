@@ -71,3 +71,36 @@ def test_build_matches_encode(handle):
         d = td.download()
         assert np.array_equal(d[:-4].reshape(-1, 4), np.array(descs[:tiles], np.int64).astype(np.int32))
         assert (d[-4:] == -1).all()
+
+
+@pytest.mark.parametrize("misaligned", [False, True])
+def test_back_to_back_calls_keep_their_order(handle, misaligned):
+    """The launches of a pointer-array batch overlap (table builder, grouped
+    kernel, the pass over flagged entries): calls queued without a wait between
+    them, each reading what the one before wrote, give the words that the same
+    calls give one at a time."""
+    n, batch, rounds = 96, 40, 12
+    rng = np.random.default_rng(3)
+    step = n * n + (1 if misaligned else 0)  # every other matrix off 16 bytes
+    mats = [hb.DeviceArray(handle, (rng.standard_normal(batch * step + 8) / 16).astype(np.float16))
+            for _ in range(3)]
+    arrs = [hb.DeviceArray(handle, np.array([m.ptr + 2 * step * i for i in range(batch)], np.uint64))
+            for m in mats]
+    start = [m.download() for m in mats]
+
+    def play(wait):
+        for m, x in zip(mats, start):
+            m.upload(x)
+        for r in range(rounds):
+            a, b, c = (arrs[(r + j) % 3] for j in range(3))
+            assert hb.gemm_batched(handle, 0, r & 1, n, n, n, 1.0, a.ptr, n, b.ptr, n, 0.5, c.ptr, n,
+                                   batch, np.float16) == 0
+            if wait:
+                assert hb.device_error(handle) == 0
+        return [m.download() for m in mats]
+
+    want = play(True)
+    for _ in range(3):
+        for g, w in zip(play(False), want):
+            assert np.array_equal(g.view(np.uint16), w.view(np.uint16))
+    assert hb.device_error(handle) == 0
