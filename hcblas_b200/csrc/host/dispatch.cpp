@@ -42,6 +42,66 @@ bool aligned16(const void *p, int64_t off, int esz) {
  * launch. */
 constexpr double REALIGN_MIN_MNK = 268435456.0; /* 2^28 */
 
+int simt_f32(HcblasB200State *st, const hcbk_gemm_args *a, void *stream, const char **path);
+
+/* SGEMM with an operand off 16 bytes, which the FP32 kernel fills in by
+ * four-byte copies at F32_ELEM_LOSS of its time: both operands as [k][mn]
+ * lines with 16-byte rows in scratch (one that is so already stays in place),
+ * where that saves more than the launch (4 us) and the copies (read and
+ * written at 4.2 TB/s) cost.  The sums run in the same order.  Above
+ * what the scratch pool keeps, under a caller's capture, over the workspace
+ * limit or without memory (HCBK_ERR_ALIGN) the operands are read in place;
+ * so they are below K = 512, where the ramps weigh more than the copies
+ * (8378^2 x 131 NT 449 us in place, 478 copied).  Measured (B200), in place
+ * against copied: 8378^2 x 1133 TN 3115 / 2902 us, NN 3227 / 2904, 8378^2 x 515
+ * NT 1486 / 1420, 4095^2 x 1023 TN 681 / 644, 2043^3 NT 395 / 388, TT 409 / 387;
+ * 2047^2 x 1023 NT 203.4 / 202.5 is the size where it begins to pay. */
+constexpr double F32_ELEM_LOSS = 0.07;
+constexpr size_t REALIGN_F32_MAX = (size_t)512 << 20;
+
+int simt_f32_realigned(HcblasB200State *st, const hcbk_gemm_args *a, double us, void *stream,
+                       const char **path) {
+  const bool ok_a = a->op_a == HCBK_OP_N && !(a->lda & 3) && aligned16(a->a, a->a_off, 4);
+  const bool ok_b = a->op_b != HCBK_OP_N && !(a->ldb & 3) && aligned16(a->b, a->b_off, 4);
+  /* pitch: whole 128-byte lines */
+  auto up32 = [](int64_t v) { return (v + 31) & ~int64_t(31); };
+  const size_t bytes_a = ok_a ? 0 : (size_t)up32(a->m) * a->k * 4;
+  const size_t bytes_b = ok_b ? 0 : (size_t)up32(a->n) * a->k * 4;
+  if (F32_ELEM_LOSS * us < 4.0 + 2.0 * (double)(bytes_a + bytes_b) / 4.2e6 ||
+      a->k < 512 || bytes_a + bytes_b > REALIGN_F32_MAX)
+    return HCBK_ERR_ALIGN;
+  char *ws = static_cast<char *>(call_scratch(st, bytes_a + bytes_b, stream));
+  if (!ws) return HCBK_ERR_ALIGN;
+  hcbk_gemm_args r = *a;
+  hcbk_realign_job jobs[2];
+  int transpose[2], count = 0;
+  if (!ok_a) {
+    const bool t = a->op_a != HCBK_OP_N;
+    transpose[count] = t;
+    jobs[count++] = {static_cast<const float *>(a->a) + a->a_off, a->lda, ws, up32(a->m),
+                     t ? a->k : a->m, t ? a->m : a->k};
+    r.op_a = HCBK_OP_N;
+    r.a = ws;
+    r.a_off = 0;
+    r.lda = up32(a->m);
+  }
+  if (!ok_b) {
+    const bool t = a->op_b == HCBK_OP_N;
+    transpose[count] = t;
+    jobs[count++] = {static_cast<const float *>(a->b) + a->b_off, a->ldb, ws + bytes_a,
+                     up32(a->n), t ? a->k : a->n, t ? a->n : a->k};
+    r.op_b = HCBK_OP_T;
+    r.b = ws + bytes_a;
+    r.b_off = 0;
+    r.ldb = up32(a->n);
+  }
+  int rc = timed_launch(st, stream, "pack.realign_f32",
+                        [&] { return hcbk_realign_f32(jobs, transpose, count, stream); });
+  if (!rc) rc = simt_f32(st, &r, stream, path);
+  call_scratch_free(ws, stream);
+  return rc;
+}
+
 /* Plain SGEMM / CGEMM: fma_gemm.cu, except where K is too short to pay for
  * its longer ramp (an unrolled loop fetched for a handful of slabs, a ring
  * filled by element copies when both operands are K-contiguous).  Measured on
@@ -74,13 +134,17 @@ int simt_f32(HcblasB200State *st, const hcbk_gemm_args *a, void *stream, const c
                          (a->a_array || (aligned16(a->a, a->a_off, 4) &&
                                          aligned16(a->b, a->b_off, 4) &&
                                          (a->batch == 1 || !((a->stride_a | a->stride_b) & 3))));
-    if (cfg.split == 1 && (a->k <= 128 || (k_contig && aligned && a->k < 1024) ||
-                           (mn_contig && !aligned)))
+    if (cfg.split == 1 && (a->k <= 128 || (k_contig && aligned && a->k < 1024)))
       return HCBK_ERR_ARGS;
     /* the 4 x 4-per-thread kernel: 5 us + 0.0425 us per k while every tile
      * has an SM, 0.0713 with two tiles on the busiest SM */
     if (tiles <= sms && 5.0 + 0.0425 * (double)a->k < us) return HCBK_ERR_ARGS;
     if (tiles <= 2 * sms && 5.0 + 0.0713 * (double)a->k < us) return HCBK_ERR_ARGS;
+    if (!aligned && a->batch == 1 && !a->a_array) {
+      rc = simt_f32_realigned(st, a, us, stream, path);
+      if (rc != HCBK_ERR_ALIGN) return rc;
+    }
+    if (cfg.split == 1 && mn_contig && !aligned) return HCBK_ERR_ARGS;
   }
   if (st->autotune) {
     /* the two tiles, with the planned split (another split would add up K in

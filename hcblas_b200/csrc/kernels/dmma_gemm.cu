@@ -1,6 +1,6 @@
 /*
  * dmma_gemm.cu -- native FP64 DGEMM on the FP64 tensor path of sm_100a
- * (warp-level mma.sync .f64, m16n8k4), the plain DGEMM of this library
+ * (warp-level mma.sync .f64, m16n8k16), the plain DGEMM of this library
  * (reference: lib/src/blas/dgemm/dgemm_*kernels*.cpp, one HCC tile kernel per
  * layout and size bucket).
  *

@@ -142,6 +142,8 @@ typedef struct hcbk_realign_job {
   int64_t inner, outer;
 } hcbk_realign_job;
 int hcbk_realign_f16(const hcbk_realign_job *jobs, int count, void *stream);
+/* f32 lines; job i with transpose[i] != 0: element e of line l to dst[e * ld_dst + l] */
+int hcbk_realign_f32(const hcbk_realign_job *jobs, const int *transpose, int count, void *stream);
 
 /* Split-BF16 SGEMM: operands already split into bf16 planes, K-major:
  * a_planes[t] is M rows x ld_a elements (row m holds op(A)(m, 0..K-1)),

@@ -265,7 +265,79 @@ __global__ void __launch_bounds__(256) realign_f16_kernel(const __grid_constant_
   }
 }
 
+/* --------------------------------------------- f32 realignment (SGEMM) -- */
+/*
+ * One operand or two as [k][mn] lines with 16-byte rows, for a kernel that
+ * copies those four floats at a time.  HBM bound; each warp takes a block of
+ * 32 x 32 floats, its 32 loads in flight before the first store, a transposed
+ * block through 32 x 33 floats of its own shared memory (no two warps meet).
+ * 2 x 8378 x 1133 floats, 152 MB read and written (B200): transposed 39.6 us
+ * (3.8 TB/s), straight 44.4.
+ */
+struct RealignF32Args {
+  hcbk_realign_job j[2];
+  int transpose[2];
+  int64_t cols[2];  /* 32-element blocks per line */
+  int64_t units[2]; /* blocks of each operand */
+};
+
+__global__ void __launch_bounds__(256)
+    realign_f32_kernel(const __grid_constant__ RealignF32Args a) {
+  __shared__ float tile[8][32][33];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int64_t warps = (int64_t)gridDim.x * 8, total = a.units[0] + a.units[1];
+  for (int64_t u = (int64_t)blockIdx.x * 8 + warp; u < total; u += warps) {
+    const int w = u >= a.units[0] ? 1 : 0;
+    const hcbk_realign_job &j = a.j[w];
+    const int64_t x = u - (w ? a.units[0] : 0), band = x / a.cols[w];
+    const int64_t l0 = band * 32, e0 = (x - band * a.cols[w]) * 32;
+    const int lines = (int)(j.outer - l0 < 32 ? j.outer - l0 : 32);
+    const int elems = (int)(j.inner - e0 < 32 ? j.inner - e0 : 32);
+    const float *s = static_cast<const float *>(j.src) + l0 * j.ld + e0 + lane;
+    float v[32];
+#pragma unroll
+    for (int i = 0; i < 32; ++i) v[i] = i < lines && lane < elems ? s[i * j.ld] : 0.0f;
+    if (a.transpose[w]) {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) tile[warp][i][lane] = v[i];
+      __syncwarp();
+      float *d = static_cast<float *>(j.dst) + e0 * j.ld_dst + l0 + lane;
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (i < elems && lane < lines) d[i * j.ld_dst] = tile[warp][lane][i];
+      __syncwarp();
+    } else {
+      float *d = static_cast<float *>(j.dst) + l0 * j.ld_dst + e0 + lane;
+#pragma unroll
+      for (int i = 0; i < 32; ++i)
+        if (i < lines && lane < elems) d[i * j.ld_dst] = v[i];
+    }
+  }
+}
+
 }  // namespace
+
+extern "C" int hcbk_realign_f32(const hcbk_realign_job *jobs, const int *transpose, int count,
+                                void *stream) {
+  if (count < 1 || count > 2) return HCBK_ERR_ARGS;
+  RealignF32Args a;
+  memset(&a, 0, sizeof(a));
+  for (int i = 0; i < count; ++i) {
+    const hcbk_realign_job &j = jobs[i];
+    if (j.inner <= 0 || j.outer <= 0 || j.ld_dst < (transpose[i] ? j.outer : j.inner) ||
+        (reinterpret_cast<uintptr_t>(j.src) & 3) || (reinterpret_cast<uintptr_t>(j.dst) & 15))
+      return HCBK_ERR_ARGS;
+    a.j[i] = j;
+    a.transpose[i] = transpose[i];
+    a.cols[i] = (j.inner + 31) / 32;
+    a.units[i] = a.cols[i] * ((j.outer + 31) / 32);
+  }
+  int64_t blocks = (a.units[0] + a.units[1] + 7) / 8;
+  const int64_t most = (int64_t)hcbk_sm_count() * 4;
+  if (blocks > most) blocks = most;
+  realign_f32_kernel<<<(unsigned)blocks, 256, 0, static_cast<cudaStream_t>(stream)>>>(a);
+  return cudaGetLastError() == cudaSuccess ? HCBK_OK : HCBK_ERR_LAUNCH;
+}
 
 extern "C" int hcbk_pack_split_bf16_complex(const hcbk_cpack_args *a, void *stream) {
   if (a->rows <= 0 || a->kdim <= 0 || a->nplanes < 1 || a->nplanes > 3) return HCBK_ERR_ARGS;
