@@ -389,6 +389,8 @@ __global__ void __launch_bounds__(DNT, DPER_SM) dmma_gemm_kernel(const __grid_co
       }
     }
     cluster_wait(); /* no rank reads this CTA's memory any more */
+    /* nor does this CTA: the arrivals above came before its reads of the sums */
+    if (p.batch > 1) __syncthreads();
   }
 }
 
@@ -632,6 +634,8 @@ zmma_gemm_kernel(const __grid_constant__ ZmmaParams p) {
       }
     }
     cluster_wait(); /* no rank reads this CTA's memory any more */
+    /* nor does this CTA: the arrivals above came before its reads of the sums */
+    if (p.batch > 1) __syncthreads();
   }
 }
 

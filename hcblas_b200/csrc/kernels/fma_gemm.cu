@@ -520,7 +520,8 @@ f32_gemm_kernel(const __grid_constant__ F32Params p) {
       }
     }
     if (split > 1) cluster_wait(); /* no rank reads this CTA's memory any more */
-    else __syncthreads();
+    /* nor does this CTA: the arrivals above came before its reads of the sums */
+    if (p.batch > 1) __syncthreads();
   }
 }
 
