@@ -35,10 +35,9 @@ bool aligned16(const void *p, int64_t off, int esz) {
 /* M N K from which HGEMM with operands that TMA cannot address copies them
  * into addressable scratch and runs on the tensor cores instead of the CUDA
  * cores.  Measured (B200, CUDA-core kernel against copy + tensor cores):
- * 645 x 645 x 647 37 against 18 us, 1133 x 777 x 1133 105 against 22,
- * 8378 x 32 x 1024 48 against 23, 8191 x 4095 x 17 109 against 53,
- * 8378 x 1133 x 777 521 against 51 (beta != 0), 4095^3 3416 against 139.
- * Smaller products keep the path that needs neither scratch nor a second
+ * 645 x 645 x 647 37 against 17 us, 8378 x 32 x 1024 48 against 23,
+ * 8191 x 4095 x 17 109 against 44, 8378 x 1133 x 777 521 against 51
+ * (beta != 0), 4095^3 3416 against 200.  Smaller products keep the path that needs neither scratch nor a second
  * launch. */
 constexpr double REALIGN_MIN_MNK = 268435456.0; /* 2^28 */
 
@@ -224,51 +223,111 @@ bool use_pair(const HcblasB200State *st, int64_t m, int64_t n, int64_t bn) {
   return tiles_of(m, n, 256, bn) >= hcbk_sm_count() / 2;
 }
 
-/* HGEMM on tcgen05 with operands read in place by TMA; an operand that TMA
- * cannot address (base or leading dimension off 16 bytes) is first copied
- * into scratch lines that it can, when the product is large enough to pay for
- * the extra pass and launch. */
+/* The tile width of a product with promoted sums (C transposed: N is its tile
+ * rows).  A wave of 128 x 256 tiles costs 1.3 to 1.5 waves of 128 x 128
+ * (B200: 8378 x 1133 x 777 3 against 5 waves, 43 / 55 us; 2047^3 1 against 2,
+ * 37 / 49; 1133 x 777 x 14521 one each, 178 / 140; 645^2 x 647 20.6 / 16.5).  CTA
+ * pairs hand each chunk of sums over between two SMs (51, 49, 140 and 16.6 us;
+ * 4095^3 217 against 201) and run only when the knob asks for them. */
+int promoted_bn(int64_t m, int64_t n) {
+  const int64_t sms = hcbk_sm_count();
+  const int64_t w256 = (tiles_of(n, m, 128, 256) + sms - 1) / sms;
+  const int64_t w128 = (tiles_of(n, m, 128, 128) + sms - 1) / sms;
+  return 7 * w256 <= 5 * w128 ? 256 : 128;
+}
+
+/* HGEMM on tcgen05, operands addressable by TMA.  promote: with promoted sums
+ * (see hgemm_realigned). */
+int hgemm_tc_run(HcblasB200State *st, const hcbk_gemm_args *a, bool promote, int *err, void *stream,
+                 const char **path) {
+  auto launch = [&](const hcbk_gemm_args *t, int bn, int pair) {
+    return promote ? hcbk_hgemm_tc_promoted(t, bn, pair, err, stream)
+                   : hcbk_hgemm_tc(t, bn, pair, err, stream);
+  };
+  int pair, bn;
+  if (promote) {
+    pair = st->tc_pair == 2 ? 1 : 0;
+    bn = pair ? 256 : promoted_bn(a->m, a->n);
+  } else {
+    pair = use_pair(st, a->m, a->n, 256) ? 1 : 0;
+    bn = pair || tiles_of(a->m, a->n, 128, 256) >= hcbk_sm_count() ? 256 : 128;
+  }
+  if (st->autotune && st->tc_pair == 1) {
+    /* candidates: 128x128, 128x256, 256x256 over a CTA pair; with beta != 0
+     * they write a scratch matrix of C's shape */
+    static const int cbn[3] = {128, 256, 256}, cpair[3] = {0, 0, 1};
+    TuneTarget tt(a, stream);
+    const int c = tune_choice(st, stream, tune_key(promote ? "hgemm_tc_sum" : "hgemm_tc", a), 3,
+                              [&](int i) {
+      const hcbk_gemm_args *t = tt.args();
+      if (!t) return (int)HCBK_ERR_NOMEM;
+      return launch(t, cbn[i], cpair[i]);
+    }, pair ? 2 : bn == 256 ? 1 : 0);
+    bn = cbn[c];
+    pair = cpair[c];
+  }
+  *path = pair ? "tc.h.256x256.pair" : bn == 256 ? "tc.h.128x256" : "tc.h.128x128";
+  return timed_launch(st, stream, *path, [&] { return launch(a, bn, pair); });
+}
+
+/* HGEMM with an operand that TMA cannot address (base or leading dimension
+ * off 16 bytes): copied into scratch lines that it can, when the product is
+ * large enough to pay for the extra pass and launch.  HCBK_ERR_ALIGN where it
+ * is not, or the scratch cannot be had: the CUDA-core kernel then reads the
+ * operands in place.  The tensor core truncates its f32 sums, that kernel
+ * rounds them: partial sums are promoted to registers, so that the same call
+ * loses no bits by its size or by the alignment of its operands. */
+int hgemm_realigned(HcblasB200State *st, const hcbk_gemm_args *a, bool ok_a, bool ok_b,
+                    void *stream, const char **path) {
+  if (st->inject_timeout || (double)a->m * (double)a->n * (double)a->k < REALIGN_MIN_MNK ||
+      a->m > 0x7fffffff || a->n > 0x7fffffff || a->k > 0x7fffffff)
+    return HCBK_ERR_ALIGN;
+  /* stored lines: `inner` contiguous elements, `outer` lines */
+  const int64_t in_a = a->op_a == HCBK_OP_N ? a->m : a->k;
+  const int64_t out_a = a->op_a == HCBK_OP_N ? a->k : a->m;
+  const int64_t in_b = a->op_b == HCBK_OP_N ? a->k : a->n;
+  const int64_t out_b = a->op_b == HCBK_OP_N ? a->n : a->k;
+  auto up8 = [](int64_t v) { return (v + 7) & ~int64_t(7); };
+  const size_t bytes_a = ok_a ? 0 : ((size_t)up8(in_a) * out_a * 2 + 255) & ~size_t(255);
+  const size_t bytes_b = ok_b ? 0 : (size_t)up8(in_b) * out_b * 2;
+  char *ws = static_cast<char *>(call_scratch(st, bytes_a + bytes_b, stream));
+  if (!ws) return HCBK_ERR_ALIGN;
+  int *err = device_error_flag(st);
+  if (!err) {
+    call_scratch_free(ws, stream);
+    return HCBK_ERR_ALIGN;
+  }
+  hcbk_gemm_args r = *a;
+  hcbk_realign_job jobs[2];
+  int count = 0;
+  if (!ok_a) {
+    jobs[count++] = {static_cast<const uint16_t *>(a->a) + a->a_off, a->lda, ws, up8(in_a),
+                     in_a, out_a};
+    r.a = ws;
+    r.a_off = 0;
+    r.lda = up8(in_a);
+  }
+  if (!ok_b) {
+    jobs[count++] = {static_cast<const uint16_t *>(a->b) + a->b_off, a->ldb, ws + bytes_a,
+                     up8(in_b), in_b, out_b};
+    r.b = ws + bytes_a;
+    r.b_off = 0;
+    r.ldb = up8(in_b);
+  }
+  int rc = timed_launch(st, stream, "pack.realign_f16",
+                        [&] { return hcbk_realign_f16(jobs, count, stream); });
+  if (!rc) rc = hgemm_tc_run(st, &r, true, err, stream, path);
+  call_scratch_free(ws, stream);
+  return rc;
+}
+
+/* HGEMM on tcgen05 with operands read in place by TMA where it can address
+ * them. */
 int hgemm_tc(HcblasB200State *st, const hcbk_gemm_args *a, void *stream, const char **path) {
   if (a->batch != 1 || a->a_array) return HCBK_ERR_ARGS;
   const bool ok_a = aligned16(a->a, a->a_off, 2) && !(a->lda & 7);
   const bool ok_b = aligned16(a->b, a->b_off, 2) && !(a->ldb & 7);
-  if (!ok_a || !ok_b) {
-    if (st->inject_timeout || (double)a->m * (double)a->n * (double)a->k < REALIGN_MIN_MNK ||
-        a->m > 0x7fffffff || a->n > 0x7fffffff || a->k > 0x7fffffff)
-      return HCBK_ERR_ALIGN;
-    /* stored lines: `inner` contiguous elements, `outer` lines */
-    const int64_t in_a = a->op_a == HCBK_OP_N ? a->m : a->k;
-    const int64_t out_a = a->op_a == HCBK_OP_N ? a->k : a->m;
-    const int64_t in_b = a->op_b == HCBK_OP_N ? a->k : a->n;
-    const int64_t out_b = a->op_b == HCBK_OP_N ? a->n : a->k;
-    auto up8 = [](int64_t v) { return (v + 7) & ~int64_t(7); };
-    const size_t bytes_a = ok_a ? 0 : ((size_t)up8(in_a) * out_a * 2 + 255) & ~size_t(255);
-    const size_t bytes_b = ok_b ? 0 : (size_t)up8(in_b) * out_b * 2;
-    char *ws = static_cast<char *>(call_scratch(st, bytes_a + bytes_b, stream));
-    if (!ws) return HCBK_ERR_ALIGN;
-    hcbk_gemm_args r = *a;
-    hcbk_realign_job jobs[2];
-    int count = 0;
-    if (!ok_a) {
-      jobs[count++] = {static_cast<const uint16_t *>(a->a) + a->a_off, a->lda, ws, up8(in_a),
-                       in_a, out_a};
-      r.a = ws;
-      r.a_off = 0;
-      r.lda = up8(in_a);
-    }
-    if (!ok_b) {
-      jobs[count++] = {static_cast<const uint16_t *>(a->b) + a->b_off, a->ldb, ws + bytes_a,
-                       up8(in_b), in_b, out_b};
-      r.b = ws + bytes_a;
-      r.b_off = 0;
-      r.ldb = up8(in_b);
-    }
-    int rc = timed_launch(st, stream, "pack.realign_f16",
-                          [&] { return hcbk_realign_f16(jobs, count, stream); });
-    if (!rc) rc = hgemm_tc(st, &r, stream, path);
-    call_scratch_free(ws, stream);
-    return rc;
-  }
+  if (!ok_a || !ok_b) return hgemm_realigned(st, a, ok_a, ok_b, stream, path);
   int *err = device_error_flag(st);
   if (!err) return HCBK_ERR_NOMEM;
   if (st->inject_timeout) { /* failure-detection test: one call, then disarmed */
@@ -279,24 +338,7 @@ int hgemm_tc(HcblasB200State *st, const hcbk_gemm_args *a, void *stream, const c
     /* a shape the injection does not accept fails the call (no fallback) */
     return rc == HCBK_ERR_ARGS || rc == HCBK_ERR_ALIGN ? HCBK_ERR_LAUNCH : rc;
   }
-  int pair = use_pair(st, a->m, a->n, 256) ? 1 : 0;
-  int bn = pair || tiles_of(a->m, a->n, 128, 256) >= hcbk_sm_count() ? 256 : 128;
-  if (st->autotune && st->tc_pair == 1) {
-    /* candidates: 128x128, 128x256, 256x256 over a CTA pair; with beta != 0
-     * they write a scratch matrix of C's shape */
-    static const int cbn[3] = {128, 256, 256}, cpair[3] = {0, 0, 1};
-    TuneTarget tt(a, stream);
-    const int c = tune_choice(st, stream, tune_key("hgemm_tc", a), 3, [&](int i) {
-      const hcbk_gemm_args *t = tt.args();
-      if (!t) return (int)HCBK_ERR_NOMEM;
-      return hcbk_hgemm_tc(t, cbn[i], cpair[i], err, stream);
-    }, pair ? 2 : bn == 256 ? 1 : 0);
-    bn = cbn[c];
-    pair = cpair[c];
-  }
-  *path = pair ? "tc.h.256x256.pair" : bn == 256 ? "tc.h.128x256" : "tc.h.128x128";
-  return timed_launch(st, stream, *path,
-                      [&] { return hcbk_hgemm_tc(a, bn, pair, err, stream); });
+  return hgemm_tc_run(st, a, false, err, stream, path);
 }
 
 /* Split-BF16 SGEMM: split both operands into bf16 planes (K-major), then one

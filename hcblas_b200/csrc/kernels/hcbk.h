@@ -122,6 +122,10 @@ int hcbk_peak_probe(int kind, int iters, double *tflops);
  * `err` is a device int that receives a nonzero code if a pipeline wait
  * times out (the kernel then exits instead of hanging). */
 int hcbk_hgemm_tc(const hcbk_gemm_args *args, int bn, int pair, int *err, void *stream);
+/* The same product with the tensor core's own sums limited to 128 K and added
+ * up in f32 registers with round-to-nearest: the error stays within that of an
+ * FP32 FMA chain over K.  Any C. */
+int hcbk_hgemm_tc_promoted(const hcbk_gemm_args *args, int bn, int pair, int *err, void *stream);
 /* Failure-detection test of the bounded pipeline waits: the HGEMM kernel on
  * one 128 x 128 tile of one K block (beta == 0) whose producer arms the
  * stage barrier without issuing its load, so that the MMA warp's wait runs

@@ -450,6 +450,17 @@ __device__ __forceinline__ void tmem_ld_32x32b_x32(uint32_t taddr, uint32_t (&r)
       : "memory");
 }
 
+__device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
+        "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+
 __device__ __forceinline__ void tmem_ld_wait() {
   asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 }
@@ -562,8 +573,9 @@ constexpr uint32_t COLS_PITCH = 2 * COLS_ROWS + 16; /* the rows + 16 bytes of al
 constexpr uint32_t COLS_WARP_BYTES = 32 * COLS_PITCH;
 
 /* whole chunks of the 32 columns at C (ldc apart; `rows` <= COLS_ROWS rows,
- * `cols` valid columns) from shared to global memory (STORE) or back */
-template <bool STORE>
+ * `cols` valid columns) from shared to global memory (STORE) or back, U chunks
+ * in flight per lane */
+template <bool STORE, int U = 8>
 __device__ __forceinline__ void cols_copy(uint8_t *buf, __half *C, long long ldc, int rows,
                                           int cols) {
   const int lane = threadIdx.x & 31;
@@ -573,12 +585,12 @@ __device__ __forceinline__ void cols_copy(uint8_t *buf, __half *C, long long ldc
   uint8_t *g = reinterpret_cast<uint8_t *>(C + (long long)j0 * ldc);
   uint8_t *s = buf + j0 * COLS_PITCH + c16;
 #pragma unroll 1
-  for (int h = 0; h < 32; h += 16) {
-    uint4 v[8];
-    uint8_t *at[8];
-    bool on[8];
+  for (int h = 0; h < 32; h += 2 * U) {
+    uint4 v[U];
+    uint8_t *at[U];
+    bool on[U];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) { /* every load before the first store */
+    for (int i = 0; i < U; ++i) { /* every load before the first store */
       const int mis = (int)(reinterpret_cast<uintptr_t>(g) & 15);
       on[i] = h + 2 * i + j0 < cols && c16 >= mis && c16 + 16 <= mis + bytes;
       at[i] = g - mis + c16;
@@ -588,9 +600,9 @@ __device__ __forceinline__ void cols_copy(uint8_t *buf, __half *C, long long ldc
                      : *reinterpret_cast<const uint4 *>(at[i]);
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int i = 0; i < U; ++i)
       if (on[i]) *reinterpret_cast<uint4 *>(STORE ? at[i] : s + 2 * i * COLS_PITCH) = v[i];
-    s += 16 * COLS_PITCH;
+    s += 2 * U * COLS_PITCH;
   }
 }
 
@@ -617,68 +629,111 @@ __device__ __forceinline__ void cols_ends(uint8_t *sb, __half *g, int rows) {
     }
 }
 
+/* The three steps of a piece of C -- `nr` <= COLS_ROWS rows of the warp's 32
+ * columns at C, `cols` of them valid, lane i holding column i -- with a
+ * __syncwarp() between them: C into the staging (beta != 0), the sums merged
+ * there, the staging to C. */
+__device__ __forceinline__ void cols_fetch(uint8_t *buf, __half *C, long long ldc, int nr,
+                                           int cols) {
+  const int lane = threadIdx.x & 31;
+  cols_copy<false>(buf, C, ldc, nr, cols);
+  if (lane < cols) cols_ends<false>(buf + lane * COLS_PITCH, C + (long long)lane * ldc, nr);
+}
+/* the same with asynchronous copies of the whole chunks (no registers, no
+ * wait): cols_fetch_wait() and a __syncwarp() before they are read */
+__device__ __forceinline__ void cols_fetch_async(uint8_t *buf, __half *C, long long ldc, int nr,
+                                                 int cols) {
+  const int lane = threadIdx.x & 31;
+  const int c16 = 16 * (lane & 15), j0 = lane >> 4;
+  const uint8_t *g = reinterpret_cast<const uint8_t *>(C + (long long)j0 * ldc);
+  uint32_t s = smem_u32(buf + j0 * COLS_PITCH + c16);
+#pragma unroll 4
+  for (int j = j0; j < 32; j += 2, g += 4 * ldc, s += 2 * COLS_PITCH) { /* two columns */
+    const int mis = (int)(reinterpret_cast<uintptr_t>(g) & 15);
+    if (j < cols && c16 >= mis && c16 + 16 <= mis + 2 * nr)
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(s), "l"(g - mis + c16)
+                   : "memory");
+  }
+  if (lane < cols) cols_ends<false>(buf + lane * COLS_PITCH, C + (long long)lane * ldc, nr);
+}
+__device__ __forceinline__ void cols_fetch_wait() {
+  asm volatile("cp.async.wait_all;" ::: "memory");
+}
+template <int U = 8>
+__device__ __forceinline__ void cols_flush(uint8_t *buf, __half *C, long long ldc, int nr,
+                                           int cols) {
+  const int lane = threadIdx.x & 31;
+  cols_copy<true, U>(buf, C, ldc, nr, cols);
+  if (lane < cols) cols_ends<true>(buf + lane * COLS_PITCH, C + (long long)lane * ldc, nr);
+}
+/* staging = alpha * sum (+ beta * staging); load(g, r) gives rows g .. g + 31
+ * of the lane's column (f32 bit patterns).  GROUPS > 0: that many groups of
+ * 32, unrolled (sums in registers). */
+template <int GROUPS, class Load>
+__device__ __forceinline__ void cols_merge(uint8_t *buf, const __half *C, long long ldc, int nr,
+                                           float alpha, float beta, bool ld_c, Load &&load) {
+  const int lane = threadIdx.x & 31;
+  const int mis = (int)(reinterpret_cast<uintptr_t>(C + (long long)lane * ldc) & 15);
+  uint32_t *w = reinterpret_cast<uint32_t *>(buf + lane * COLS_PITCH + (mis & ~3));
+  const uint32_t sft = (mis & 2) * 8; /* 16 when the column starts in a word's upper half */
+  uint32_t carry = ld_c ? w[0] : 0u, old = carry;
+#pragma unroll(GROUPS > 0 ? GROUPS : 1)
+  for (int g = 0; g < (GROUPS > 0 ? 32 * GROUPS : nr); g += 32) {
+    if (g >= nr) continue;
+    uint32_t r[32];
+    load(g, r);
+    uint32_t *wg = w + g / 2;
+    if (ld_c) {
+#pragma unroll
+      for (int i = 0; i < 16; ++i) {
+        /* rows 2i, 2i + 1 of the group: words i and i + 1 of the column */
+        const uint32_t next = wg[i + 1];
+        const uint32_t c2 = __funnelshift_r(old, next, sft);
+        old = next;
+        const __half2 h = *reinterpret_cast<const __half2 *>(&c2);
+        r[2 * i] = __float_as_uint(
+            fmaf(beta, __low2float(h), alpha * __uint_as_float(r[2 * i])));
+        r[2 * i + 1] = __float_as_uint(
+            fmaf(beta, __high2float(h), alpha * __uint_as_float(r[2 * i + 1])));
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(alpha * __uint_as_float(r[i]));
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const __half2 h =
+          __floats2half2_rn(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
+      const uint32_t hw = *reinterpret_cast<const uint32_t *>(&h);
+      wg[i] = __funnelshift_l(carry, hw, sft);
+      carry = hw;
+    }
+    /* the last row of a shifted column; the next group rewrites the word */
+    if (!ld_c || g + 32 >= nr) wg[16] = __funnelshift_l(carry, 0u, sft);
+  }
+}
+
 /* One warp's 32 columns x `width` rows of C: TMEM lane i (of this warp) is
  * column i, `width` TMEM columns at tbase are consecutive rows; rows / cols
  * valid; C the first of them.  C = alpha * acc (+ beta * C). */
 __device__ __forceinline__ void cols_tile(uint8_t *buf, uint32_t tbase, int width, __half *C,
                                           long long ldc, int rows, int cols, float alpha,
                                           float beta, bool ld_c) {
-  const int lane = threadIdx.x & 31;
-  uint8_t *sb = buf + lane * COLS_PITCH;
   if (rows > width) rows = width;
 #pragma unroll 1
   for (int r0 = 0; r0 < rows; r0 += COLS_ROWS) {
     const int nr = rows - r0 < COLS_ROWS ? rows - r0 : COLS_ROWS;
-    __half *Cp = C + r0;
-    __half *col = Cp + (long long)lane * ldc;
-    const int mis = (int)(reinterpret_cast<uintptr_t>(col) & 15);
-    uint32_t *w = reinterpret_cast<uint32_t *>(sb + (mis & ~3));
-    const uint32_t sft = (mis & 2) * 8; /* 16 when the column starts in a word's upper half */
     __syncwarp(); /* the previous rows have been copied out */
     if (ld_c) {
-      cols_copy<false>(buf, Cp, ldc, nr, cols);
-      if (lane < cols) cols_ends<false>(sb, col, nr);
+      cols_fetch(buf, C + r0, ldc, nr, cols);
       __syncwarp();
     }
-    uint32_t carry = ld_c ? w[0] : 0u, old = carry;
-#pragma unroll 1
-    for (int g = 0; g < nr; g += 32) {
-      uint32_t r[32];
+    cols_merge<0>(buf, C + r0, ldc, nr, alpha, beta, ld_c, [&](int g, uint32_t(&r)[32]) {
       tmem_ld_32x32b_x32(tbase + r0 + g, r);
       tmem_ld_wait();
-      uint32_t *wg = w + g / 2;
-      if (ld_c) {
-#pragma unroll
-        for (int i = 0; i < 16; ++i) {
-          /* rows 2i, 2i + 1 of the group: words i and i + 1 of the column */
-          const uint32_t next = wg[i + 1];
-          const uint32_t c2 = __funnelshift_r(old, next, sft);
-          old = next;
-          const __half2 h = *reinterpret_cast<const __half2 *>(&c2);
-          r[2 * i] = __float_as_uint(
-              fmaf(beta, __low2float(h), alpha * __uint_as_float(r[2 * i])));
-          r[2 * i + 1] = __float_as_uint(
-              fmaf(beta, __high2float(h), alpha * __uint_as_float(r[2 * i + 1])));
-        }
-      } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i)
-          r[i] = __float_as_uint(alpha * __uint_as_float(r[i]));
-      }
-#pragma unroll
-      for (int i = 0; i < 16; ++i) {
-        const __half2 h =
-            __floats2half2_rn(__uint_as_float(r[2 * i]), __uint_as_float(r[2 * i + 1]));
-        const uint32_t hw = *reinterpret_cast<const uint32_t *>(&h);
-        wg[i] = __funnelshift_l(carry, hw, sft);
-        carry = hw;
-      }
-      /* the last row of a shifted column; the next group rewrites the word */
-      if (!ld_c || g + 32 >= nr) wg[16] = __funnelshift_l(carry, 0u, sft);
-    }
+    });
     __syncwarp();
-    cols_copy<true>(buf, Cp, ldc, nr, cols);
-    if (lane < cols) cols_ends<true>(sb, col, nr);
+    cols_flush(buf, C + r0, ldc, nr, cols);
   }
 }
 

@@ -365,6 +365,76 @@ template <int EW> struct EpiColsH {
   }
 };
 
+/* The same C from sums that are promoted.  The tensor core truncates its f32
+ * sums, which over a long K costs more bits than an FP32 FMA chain does, so its
+ * own sums span SUM_KB slabs of K and are added in registers with
+ * round-to-nearest.  Outputs that are not the correctly rounded ones, operands
+ * U[-1, 1), 1133 x 777 (FP32 FMA chain / truncated over all of K / SUM_KB = 2 /
+ * 4): K = 777 0.23 / 0.41 / 0.10 / 0.17 %, K = 4095 0.50 / 1.73 / 0.12 / 0.19 %,
+ * K = 14521 0.87 / 5.1 / 0.14 / 0.18 %; K = 129 0.09 in every column.  With
+ * operands in [0, 1) K = 2047 0.07 / 1.7 / 0.07 / 0.17 %: SUM_KB = 2.
+ *
+ * Each drain of a chunk costs the hand-over between epilogue and MMA issuer
+ * more than its loads and adds (4095^3 unpromoted 143 us, 201 promoted, 190 with
+ * the drains left out).  C (beta != 0) is copied into the staging
+ * asynchronously from the tile's start on, and the staging leaves two chunks
+ * at a time: with more in flight the 128 sums per thread spill (168 registers:
+ * 217 -> 292 us on CTA pairs). */
+constexpr int SUM_KB = 2;
+struct EpiColsSumH {
+  static constexpr bool INPLACE = false;
+  static constexpr bool PLANE_BATCH = false;
+  static constexpr int EPI_WARPS = 8;
+  static constexpr uint32_t OUT_WARP_BYTES = COLS_WARP_BYTES;
+  static constexpr uint32_t OUT_SMEM = EPI_WARPS * OUT_WARP_BYTES;
+  using AccT = float;
+
+  template <int BN>
+  static __device__ __forceinline__ void prefetch_c(const TcParams &p, int m0, int n0,
+                                                    OutStage &os) {
+    __syncwarp(); /* the last tile has been copied out */
+    const int rows = p.n - n0 < BN ? p.n - n0 : BN;
+    if (p.beta_nonzero && rows > 0)
+      cols_fetch_async(os.box, static_cast<__half *>(p.c) + n0 + (long long)m0 * p.ldc, p.ldc,
+                       rows, p.m - m0);
+  }
+
+  /* acc[j] += TMEM column j, 16 columns at a time (168 registers a thread) */
+  template <int BN, int NACC>
+  static __device__ __forceinline__ void accumulate(const TcParams &, uint32_t tbase,
+                                                    float (&acc)[BN], int /* chunk */) {
+    static_assert(NACC == 1, "one accumulator");
+#pragma unroll
+    for (int c = 0; c < BN; c += 16) {
+      uint32_t r[16];
+      tmem_ld_32x32b_x16(tbase + c, r);
+      tmem_ld_wait();
+#pragma unroll
+      for (int j = 0; j < 16; ++j) acc[c + j] += __uint_as_float(r[j]);
+    }
+  }
+
+  template <int BN>
+  static __device__ __forceinline__ void store_acc(const TcParams &p, const float (&acc)[BN], int m,
+                                                   int n0, OutStage &os) {
+    static_assert(BN <= COLS_ROWS, "one piece");
+    const int m0 = m - (int)(threadIdx.x & 31), rows = p.n - n0 < BN ? p.n - n0 : BN;
+    if (rows <= 0) return;
+    __half *C = static_cast<__half *>(p.c) + n0 + (long long)m0 * p.ldc;
+    if (p.beta_nonzero) {
+      cols_fetch_wait();
+      __syncwarp();
+    }
+    cols_merge<BN / 32>(os.box, C, p.ldc, rows, p.alpha, p.beta, p.beta_nonzero != 0,
+                        [&](int g, uint32_t(&r)[32]) {
+#pragma unroll
+                          for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(acc[g + j]);
+                        });
+    __syncwarp();
+    cols_flush<2>(os.box, C, p.ldc, rows, p.m - m0);
+  }
+};
+
 /* Modular epilogue of the CRT scheme, reducing in place in TMEM.
  * With f16 residues |r| <= 127 (moduli <= 255) the tensor core's f32 sums
  * are exact integers while below 2^24: 1024 * 127^2 + 1.5 * 255 < 2^24.
@@ -691,6 +761,15 @@ __device__ __forceinline__ WorkItem work_item(int i, int tile0, int step, int nt
   return WorkItem{tile0 + lt * step, i - lt * nchunks, 0};
 }
 
+/* the item after w of a CTA whose tiles come one after the other (w.c = -1
+ * before the first): no division per chunk */
+__device__ __forceinline__ void next_item(WorkItem &w, int step, int nchunks) {
+  if (++w.c == nchunks) {
+    w.c = 0;
+    w.t += step;
+  }
+}
+
 /* Tile order within a plane: bands of TILE_GROUP tile rows, walked column
  * by column and down each column inside the band, so that the tiles running
  * at the same time (one per SM or SM pair) cover about TILE_GROUP row tiles
@@ -729,8 +808,9 @@ __global__ void __launch_bounds__(64 + 32 * EpiWarps<EPI>::value, 1)
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(tempty + 2);
   uint64_t *obar = tempty + 4; /* output staging: two C-load barriers per epilogue warp */
   constexpr int EW = EpiWarps<EPI>::value;
-  static_assert(EW == 4 || (EW == 8 && PROMOTE_KB == 0 && !EPI::INPLACE && BN % 128 == 0),
-                "eight epilogue warps split the columns of a tile that is read once");
+  static_assert(EW == 4 || (EW == 8 && !EPI::INPLACE && BN % 128 == 0 &&
+                            (PROMOTE_KB == 0 || R::NACC == 1)),
+                "eight epilogue warps split the columns of one accumulator");
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -793,12 +873,18 @@ __global__ void __launch_bounds__(64 + 32 * EpiWarps<EPI>::value, 1)
       int s = 0;
       uint32_t ph = 0;
       bool ok = true;
+      WorkItem w{tile0, -1, 0};
+      TileMN tc_{0, 0};
+      int plane = 0;
       for (int i = 0; ok && i < nitems; ++i) {
-        const WorkItem w = work_item(i, tile0, tile_step, ntiles_local, nchunks, PAIRS);
-        const int t = w.t;
-        const int plane = EPI::PLANE_BATCH ? t / tiles_per_plane : 0;
-        const int tt = t - plane * tiles_per_plane;
-        const TileMN tc_ = tile_mn(tt, p.tiles_m, p.tiles_n);
+        if (PAIRS)
+          w = work_item(i, tile0, tile_step, ntiles_local, nchunks, PAIRS);
+        else
+          next_item(w, tile_step, nchunks);
+        if (PAIRS || w.c == 0) { /* a new tile */
+          plane = EPI::PLANE_BATCH ? w.t / tiles_per_plane : 0;
+          tc_ = tile_mn(w.t - plane * tiles_per_plane, p.tiles_m, p.tiles_n);
+        }
         const int tm = tc_.m, tn = tc_.n;
         const int row0 = (tm * CG + (int)rank) * BM;               /* this CTA's A rows */
         const int col0 = tn * BN + (int)rank * (int)Cfg::B_ROWS;   /* this CTA's B rows */
@@ -903,9 +989,13 @@ __global__ void __launch_bounds__(64 + 32 * EpiWarps<EPI>::value, 1)
       int ci = 0; /* chunk counter (all tiles): selects the TMEM buffer */
       uint32_t uses = 0u; /* in-place mode: bit b = parity of buffer b's acquisitions */
       bool ok = true;
+      WorkItem w{tile0, -1, 0};
       for (int i = 0; ok && i < nitems; ++i, ++ci) {
         {
-          const WorkItem w = work_item(i, tile0, tile_step, ntiles_local, nchunks, PAIRS);
+          if (PAIRS)
+            w = work_item(i, tile0, tile_step, ntiles_local, nchunks, PAIRS);
+          else
+            next_item(w, tile_step, nchunks);
           const int kc = w.c * chunk_kb;
           /* in-place mode: chunk c of a tile accumulates into its slot's
            * buffer on top of the epilogue's reduced value of chunk c - 1 */
@@ -1044,9 +1134,9 @@ __global__ void __launch_bounds__(64 + 32 * EpiWarps<EPI>::value, 1)
         __syncwarp();
         release(b);
       } else {
-        typename EPI::AccT acc[BN];
+        typename EPI::AccT acc[COLS];
 #pragma unroll
-        for (int j = 0; j < BN; ++j) acc[j] = 0;
+        for (int j = 0; j < COLS; ++j) acc[j] = 0;
         for (int kc = 0; kc < kblocks; kc += chunk_kb, ++ci) {
           const int b = ci % NBUF;
           const uint32_t tph = (ci / NBUF) & 1;
@@ -1055,17 +1145,19 @@ __global__ void __launch_bounds__(64 + 32 * EpiWarps<EPI>::value, 1)
             break;
           }
           tc_fence_after();
-          EPI::template accumulate<BN, R::NACC>(
-              p, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + b * Cfg::ACC_COLS, acc,
-              kc / chunk_kb);
+          EPI::template accumulate<COLS, R::NACC>(
+              p, tmem_base + (static_cast<uint32_t>(q * 32) << 16) + b * Cfg::ACC_COLS +
+                     half * COLS,
+              acc, kc / chunk_kb);
           tc_fence_before();
           __syncwarp();
           release(b);
         }
-        if (ok) EPI::template store_acc<BN>(p, acc, m, tn * BN, ostage);
+        if (ok) EPI::template store_acc<COLS>(p, acc, m, tn * BN + half * COLS, ostage);
       }
     }
     }
+    if constexpr (PROMOTE_KB > 0 && EW == 8) cols_fetch_wait(); /* after a failed wait */
     if constexpr (Cfg::OUT_BYTES > 0) {
       if (lane == 0) {
         /* C loads still in flight (only after a failed wait): give them a
@@ -1243,15 +1335,16 @@ extern "C" int hcbk_encode_out_2d(void *map, void *base, uint64_t rows, uint64_t
                       rows, cols, ld);
 }
 
-template <int BN, int STAGES, int EW, int CG> static int launch_cols(TcParams &p, void *stream) {
-  static_assert(TcCfg<BN, STAGES, RecipeSingle, 0, 2, CG, EpiColsH<EW>::OUT_SMEM>::OUT_BYTES > 0,
+template <int BN, int STAGES, class EPI, int CG, int PROMOTE_KB = 0>
+static int launch_cols(TcParams &p, void *stream) {
+  static_assert(TcCfg<BN, STAGES, RecipeSingle, 0, 2, CG, EPI::OUT_SMEM>::OUT_BYTES > 0,
                 "the columns' staging fits beside the stages");
-  return launch_tc<BN, STAGES, RecipeSingle, 0, EpiColsH<EW>, 0, 2, CG>(p, stream);
+  return launch_tc<BN, STAGES, RecipeSingle, 0, EPI, PROMOTE_KB, 2, CG>(p, stream);
 }
 
 /* f16 operands straight from the caller's matrices (column-major canonical). */
 static int hgemm_tc_impl(const hcbk_gemm_args *a, int bn, int pair, int *err, void *stream,
-                         int inject_skip_load) {
+                         int inject_skip_load, bool promote) {
   if (a->dtype != HCBK_H || a->batch != 1 || a->a_array || a->op_a == HCBK_OP_C ||
       a->op_b == HCBK_OP_C)
     return HCBK_ERR_ARGS;
@@ -1270,7 +1363,7 @@ static int hgemm_tc_impl(const hcbk_gemm_args *a, int bn, int pair, int *err, vo
    * product C^T = op(B)^T op(A)^T, whose epilogue holds C by columns */
   p.out_tma =
       make_map_out(&p.tc, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, p.c, a->m, a->n, a->ldc) == HCBK_OK;
-  const bool swap = !p.out_tma && !inject_skip_load;
+  const bool swap = (promote || !p.out_tma) && !inject_skip_load;
   p.m = (int)(swap ? a->n : a->m);
   p.n = (int)(swap ? a->m : a->n);
   p.k = (int)a->k;
@@ -1305,6 +1398,11 @@ static int hgemm_tc_impl(const hcbk_gemm_args *a, int bn, int pair, int *err, vo
       return HCBK_ERR_ARGS;
     p.inject_skip_load = 1;
   }
+  if (promote) {
+    if (pair) return launch_cols<256, 4, EpiColsSumH, 2, SUM_KB>(p, stream);
+    if (bn == 256) return launch_cols<256, 3, EpiColsSumH, 1, SUM_KB>(p, stream);
+    return launch_cols<128, 4, EpiColsSumH, 1, SUM_KB>(p, stream);
+  }
   if (swap) {
     /* fewer stages: the columns' staging takes their place.  Eight epilogue
      * warps where the epilogue bounds the tile, four where its MMAs do;
@@ -1312,13 +1410,13 @@ static int hgemm_tc_impl(const hcbk_gemm_args *a, int bn, int pair, int *err, vo
      * 8378 x 1133 x 777 beta != 0 50 against 57, beta == 0 41 both,
      * 4095^3 149 against 140. */
     if (p.k <= (p.beta_nonzero ? 1024 : 512)) {
-      if (pair) return launch_cols<256, 4, 8, 2>(p, stream);
-      if (bn == 256) return launch_cols<256, 3, 8, 1>(p, stream);
-      return launch_cols<128, 4, 8, 1>(p, stream);
+      if (pair) return launch_cols<256, 4, EpiColsH<8>, 2>(p, stream);
+      if (bn == 256) return launch_cols<256, 3, EpiColsH<8>, 1>(p, stream);
+      return launch_cols<128, 4, EpiColsH<8>, 1>(p, stream);
     }
-    if (pair) return launch_cols<256, 5, 4, 2>(p, stream);
-    if (bn == 256) return launch_cols<256, 3, 4, 1>(p, stream);
-    return launch_cols<128, 5, 4, 1>(p, stream);
+    if (pair) return launch_cols<256, 5, EpiColsH<4>, 2>(p, stream);
+    if (bn == 256) return launch_cols<256, 3, EpiColsH<4>, 1>(p, stream);
+    return launch_cols<128, 5, EpiColsH<4>, 1>(p, stream);
   }
   if (pair) return launch_tc<256, 6, RecipeSingle, 0, EH, 0, 2, 2>(p, stream);
   if (bn == 256) return launch_tc<256, 4, RecipeSingle, 0, EH>(p, stream);
@@ -1326,11 +1424,16 @@ static int hgemm_tc_impl(const hcbk_gemm_args *a, int bn, int pair, int *err, vo
 }
 
 extern "C" int hcbk_hgemm_tc(const hcbk_gemm_args *a, int bn, int pair, int *err, void *stream) {
-  return hgemm_tc_impl(a, bn, pair, err, stream, 0);
+  return hgemm_tc_impl(a, bn, pair, err, stream, 0, false);
+}
+
+extern "C" int hcbk_hgemm_tc_promoted(const hcbk_gemm_args *a, int bn, int pair, int *err,
+                                      void *stream) {
+  return hgemm_tc_impl(a, bn, pair, err, stream, 0, true);
 }
 
 extern "C" int hcbk_hgemm_tc_inject_timeout(const hcbk_gemm_args *a, int *err, void *stream) {
-  return hgemm_tc_impl(a, 128, 0, err, stream, 1);
+  return hgemm_tc_impl(a, 128, 0, err, stream, 1, false);
 }
 
 /* split-BF16 SGEMM on pre-split K-major planes:
