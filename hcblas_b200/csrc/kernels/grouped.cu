@@ -62,7 +62,7 @@ struct GCfg {
 struct Params {
   const hcbk_grouped_entry *table;
   const int32_t *tile_start;
-  const int4 *tile_desc; /* per tile: problem | flags << 24, tm, tn, k (host tables) */
+  const int4 *tile_desc; /* per tile: problem | flags << 24, tm, tn, k */
   int count;
   int total_tiles;
   /* uniform batches (device-built tables): every problem has uniform_tiles
@@ -92,18 +92,21 @@ struct TileRef {
   int flags; /* HCBK_GT_* */
 };
 
-/* One 16-byte load per tile (host tables) or arithmetic (uniform batches):
- * a binary search over the tile prefix sums costs a dozen dependent global
- * loads per tile and role, which dominated small tiles. */
+/* One 16-byte load per tile or arithmetic (uniform batches): a binary search
+ * over the tile prefix sums costs a dozen dependent global loads per tile and
+ * role, which dominated small tiles.  Ordinary loads here and in epi_ref: the
+ * kernel is launched while the table's builder may still write, so that the
+ * read-only path (memory that nobody writes during the kernel's life) is not
+ * open to it, and only ordinary accesses keep their place behind
+ * grid_dependency_wait(). */
 __device__ __forceinline__ TileRef tile_ref(const Params &p, int t) {
   if (p.uniform_tiles > 0) {
     const int g = t / p.uniform_tiles, lt = t - g * p.uniform_tiles;
     const hcbk_grouped_entry *e = p.table + g;
-    const int flags = p.u_flags | (__ldg(&e->c_tma) ? HCBK_GT_CTMA : 0) |
-                      (__ldg(&e->skip) ? HCBK_GT_SKIP : 0);
+    const int flags = p.u_flags | (e->c_tma ? HCBK_GT_CTMA : 0) | (e->skip ? HCBK_GT_SKIP : 0);
     return TileRef{e, lt % p.u_tiles_m, lt / p.u_tiles_m, p.u_k, flags};
   }
-  const int4 d = __ldg(p.tile_desc + t);
+  const int4 d = p.tile_desc[t];
   return TileRef{p.table + (d.x & 0xffffff), d.y, d.z, d.w, (int)((unsigned)d.x >> 24)};
 }
 
@@ -118,9 +121,9 @@ struct EpiRef {
 __device__ __forceinline__ EpiRef epi_ref(const Params &p, int t) {
   EpiRef x;
   x.r = tile_ref(p, t);
-  x.m = __ldg(&x.r.e->m);
-  x.n = __ldg(&x.r.e->n);
-  x.ldc = __ldg(&x.r.e->ldc);
+  x.m = x.r.e->m;
+  x.n = x.r.e->n;
+  x.ldc = x.r.e->ldc;
   x.c = x.r.e->c;
   return x;
 }
