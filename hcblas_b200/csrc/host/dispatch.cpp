@@ -148,11 +148,15 @@ int simt_f32(HcblasB200State *st, const hcbk_gemm_args *a, void *stream, const c
   if (st->autotune) {
     /* the two tiles, with the planned split (another split would add up K in
      * another order); beta == 0: the candidates write C, which the final
-     * launch rewrites, otherwise a scratch matrix of C's shape */
+     * launch rewrites, otherwise a scratch matrix of C's shape.  A family of
+     * its own per split: calls of one size bucket may also go to
+     * simt_gemm.cu, or be split otherwise. */
     const bool zero_beta = a->beta_re == 0.0 && a->beta_im == 0.0;
     TuneTarget tt(a, stream);
+    char family[24];
+    std::snprintf(family, sizeof(family), "simt|fma.k%d", cfg.split);
     if (zero_beta || tt.usable())
-      cfg.tile = tune_choice(st, stream, tune_key("simt", a), 2, [&](int i) {
+      cfg.tile = tune_choice(st, stream, tune_key(family, a), 2, [&](int i) {
         const hcbk_gemm_args *t = zero_beta ? a : tt.args();
         if (!t) return (int)HCBK_ERR_NOMEM;
         hcbk_f32_cfg c = cfg;
@@ -257,8 +261,10 @@ int hgemm_tc_run(HcblasB200State *st, const hcbk_gemm_args *a, bool promote, int
      * they write a scratch matrix of C's shape */
     static const int cbn[3] = {128, 256, 256}, cpair[3] = {0, 0, 1};
     TuneTarget tt(a, stream);
-    const int c = tune_choice(st, stream, tune_key(promote ? "hgemm_tc_sum" : "hgemm_tc", a), 3,
-                              [&](int i) {
+    /* a C that tensor stores cannot write takes another epilogue */
+    const bool c_boxes = aligned16(a->c, a->c_off, 2) && !((a->ldc | a->m) & 7);
+    const char *family = promote ? "hgemm_tc.sum" : c_boxes ? "hgemm_tc" : "hgemm_tc.cols";
+    const int c = tune_choice(st, stream, tune_key(family, a), 3, [&](int i) {
       const hcbk_gemm_args *t = tt.args();
       if (!t) return (int)HCBK_ERR_NOMEM;
       return launch(t, cbn[i], cpair[i]);

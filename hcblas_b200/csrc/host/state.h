@@ -14,7 +14,7 @@
 #include <vector>
 
 /* library version: hcblasGetVersionString, and part of every autotune key */
-#define HCBLAS_B200_VERSION "0.2.0"
+#define HCBLAS_B200_VERSION "0.3.0"
 
 /* one timed kernel launch (events recorded on the launch stream) */
 struct HcblasProfRec {
