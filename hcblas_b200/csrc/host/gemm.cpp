@@ -43,7 +43,10 @@ static bool is_complex(int dtype) { return dtype == HCBK_C || dtype == HCBK_Z; }
 /* Replay a captured CUDA graph of an identical earlier call, or run the call
  * eagerly and capture its launch sequence for the next time.  The capture
  * happens after the eager run, so every buffer, tensor map and attribute it
- * needs already exists and nothing is allocated while capturing. */
+ * needs already exists and nothing is allocated while capturing.  A call that
+ * took scratch of its own is remembered as one to run eagerly (exec null): a
+ * graph would hold the scratch outside the handle's pool and past a change of
+ * the workspace limit. */
 int dispatch_with_graph(HcblasB200State *st, const hcbk_gemm_args *a, void *stream,
                         const char **path) {
   int dev = 0;
@@ -58,6 +61,7 @@ int dispatch_with_graph(HcblasB200State *st, const hcbk_gemm_args *a, void *stre
   std::memcpy(key.data() + sizeof(*a) + sizeof(knobs), &stream, sizeof(stream));
   for (auto &e : st->graph_cache) {
     if (e.key == key) {
+      if (!e.exec) return dispatch_gemm(st, a, stream, path);
       if (cudaGraphLaunch(static_cast<cudaGraphExec_t>(e.exec), static_cast<cudaStream_t>(stream)) !=
           cudaSuccess) {
         cudaGetLastError();
@@ -68,8 +72,26 @@ int dispatch_with_graph(HcblasB200State *st, const hcbk_gemm_args *a, void *stre
       return HCBK_OK;
     }
   }
+  auto remember = [&](void *exec, long long launches) {
+    if (st->graph_cache.size() >= 16) {
+      if (void *first = st->graph_cache.front().exec)
+        cudaGraphExecDestroy(static_cast<cudaGraphExec_t>(first));
+      st->graph_cache.erase(st->graph_cache.begin());
+    }
+    HcblasGraphEntry e;
+    e.key = key;
+    e.exec = exec;
+    e.launches = launches;
+    e.path = *path;
+    st->graph_cache.push_back(std::move(e));
+  };
+  const long long scratch = call_scratch_count();
   int rc = dispatch_gemm(st, a, stream, path);
   if (rc != HCBK_OK) return rc;
+  if (call_scratch_count() != scratch) {
+    remember(nullptr, 0);
+    return HCBK_OK;
+  }
   const unsigned epoch = st->workspace_epoch;
   const long long before = launch_count();
   cudaStream_t cs = static_cast<cudaStream_t>(stream);
@@ -78,9 +100,7 @@ int dispatch_with_graph(HcblasB200State *st, const hcbk_gemm_args *a, void *stre
     return HCBK_OK;
   }
   const char *p2 = nullptr;
-  st->own_capture = stream;
   const int rc2 = dispatch_gemm(st, a, stream, &p2);
-  st->own_capture = nullptr;
   cudaGraph_t graph = nullptr;
   const cudaError_t ce = cudaStreamEndCapture(cs, &graph);
   const long long captured = launch_count() - before;
@@ -88,16 +108,7 @@ int dispatch_with_graph(HcblasB200State *st, const hcbk_gemm_args *a, void *stre
   cudaGraphExec_t exec = nullptr;
   if (rc2 == HCBK_OK && ce == cudaSuccess && graph && st->workspace_epoch == epoch &&
       cudaGraphInstantiate(&exec, graph, 0) == cudaSuccess) {
-    if (st->graph_cache.size() >= 16) {
-      cudaGraphExecDestroy(static_cast<cudaGraphExec_t>(st->graph_cache.front().exec));
-      st->graph_cache.erase(st->graph_cache.begin());
-    }
-    HcblasGraphEntry e;
-    e.key = key;
-    e.exec = exec;
-    e.launches = captured;
-    e.path = *path;
-    st->graph_cache.push_back(std::move(e));
+    remember(exec, captured);
   } else {
     cudaGetLastError();
   }

@@ -113,6 +113,9 @@ void *ensure_workspace(HcblasB200State *st, size_t bytes, void *stream_v) {
   return p;
 }
 
+static thread_local long long t_scratch_calls = 0;
+long long call_scratch_count() { return t_scratch_calls; }
+
 void *call_scratch(HcblasB200State *st, size_t bytes, void *stream_v) {
   cudaStream_t stream = static_cast<cudaStream_t>(stream_v);
   if (st->workspace_limit && bytes > st->workspace_limit) return nullptr;
@@ -124,8 +127,7 @@ void *call_scratch(HcblasB200State *st, size_t bytes, void *stream_v) {
     cudaGetLastError();
     return nullptr;
   }
-  if (cap != cudaStreamCaptureStatusNone && (!stream_v || st->own_capture != stream_v))
-    return nullptr;
+  if (cap != cudaStreamCaptureStatusNone) return nullptr;
   cudaMemPool_t pool;
   {
     std::lock_guard<std::mutex> lock(st->scratch_mutex);
@@ -152,6 +154,7 @@ void *call_scratch(HcblasB200State *st, size_t bytes, void *stream_v) {
     cudaGetLastError();
     return nullptr;
   }
+  ++t_scratch_calls;
   return p;
 }
 

@@ -86,8 +86,6 @@ struct HcblasB200State {
   /* per-device memory pools of call_scratch (created on first use) */
   std::mutex scratch_mutex;
   void *scratch_pool[16] = {nullptr}; /* cudaMemPool_t */
-  /* the stream whose calls the library itself is capturing (graphs knob) */
-  void *own_capture = nullptr;
   /* device error block of the tensor-core kernels: int 0 is set when a
    * pipeline wait times out, ints 2-3 hold the wait limit in ns */
   int *dev_err = nullptr;
@@ -178,12 +176,14 @@ void *ensure_workspace(HcblasB200State *st, size_t bytes, void *stream);
  * pool and handed back with call_scratch_free after the call's last launch, so
  * calls on different streams (or from different threads) never share a buffer
  * and never wait for one another.  The pool keeps up to 512 MiB between calls
- * and is given back with the handle.  nullptr while the caller captures
- * `stream` (the memory would belong to the caller's graph), beyond the
- * "workspace_mb" limit, or when the allocation fails: the caller then takes a
- * path that needs no scratch. */
+ * and is given back with the handle.  nullptr while `stream` is being captured
+ * (the memory would belong to the graph), beyond the "workspace_mb" limit, or
+ * when the allocation fails: the caller then takes a path that needs no
+ * scratch. */
 void *call_scratch(HcblasB200State *st, size_t bytes, void *stream);
 void call_scratch_free(void *p, void *stream);
+/* allocations that the calling thread has had from call_scratch */
+long long call_scratch_count();
 
 /* The handle's device error flag on the current device (allocated and
  * zeroed on first use); nullptr if it cannot be allocated. */

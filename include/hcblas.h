@@ -486,7 +486,9 @@ hcblasStatus_t hcblasPlanEmulation(int mode, int param, int bits, int dtype, lon
  *                       non-default stream) replays a CUDA graph captured
  *                       from the earlier call's launch sequence instead of
  *                       launching each kernel; 0 (default) launches directly.
- *                       Graphs are dropped when the handle's workspace moves.
+ *                       Graphs are dropped when the handle's workspace moves;
+ *                       calls that copy their operands (see "workspace_mb")
+ *                       are always launched directly.
  *   "tc_pair"           tensor-core paths (HGEMM, split-BF16, CRT): CTA-pair
  *                       kernels (tcgen05 cta_group::2, 256-row tiles over two
  *                       SMs): 0 never, 1 when the problem fills every SM pair
@@ -523,6 +525,15 @@ hcblasStatus_t hcblasPlanEmulation(int mode, int param, int bits, int dtype, lon
  *                       cudaFreeAsync on the call's stream); it cannot grow
  *                       while that stream is being captured (the call then
  *                       fails the same way).
+ *                       Native HGEMM (M N K >= 2^28) and SGEMM (K >= 512)
+ *                       with operands off 16 bytes copy these into
+ *                       stream-ordered scratch beside the workspace, from a
+ *                       pool that keeps up to 512 MiB per device until the
+ *                       handle is destroyed.  The limit holds for each call's
+ *                       copies by themselves; where they would exceed it,
+ *                       while the stream is being captured, or without memory
+ *                       the call runs more slowly on the operands in place
+ *                       (the same sums in SGEMM, another order in HGEMM).
  *   "wait_timeout_us"   limit of every bounded pipeline wait in the
  *                       tensor-core kernels, in microseconds (0, the default:
  *                       2 s).  A wait that runs out records its code in the

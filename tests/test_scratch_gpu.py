@@ -1,0 +1,53 @@
+"""The scratch of calls that copy their operands: its limit under the graphs
+knob, streams that do not wait for one another, and captures on other streams."""
+import numpy as np
+import pytest
+import torch
+
+import hcblas_b200 as hb
+
+pytestmark = pytest.mark.gpu
+
+
+class Product:
+    """An HGEMM with odd leading dimensions (integers: every word is known)."""
+
+    def __init__(self, seed, M=801, N=803, K=805):
+        rng = np.random.default_rng(seed)
+        self.shape = M, N, K
+        self.a, self.b = (rng.integers(-2, 3, s).astype(np.float16) for s in ((K, M), (N, K)))
+        self.want = (self.b.astype(np.float64) @ self.a).astype(np.float16)
+
+    def upload(self, h):
+        self.d = [hb.DeviceArray(h, x.ravel()) for x in (self.a, self.b, np.zeros_like(self.want))]
+
+    def run(self, h):
+        M, N, K = self.shape
+        return hb.lib_gemm(h, hb.ColMajor, "n", "n", M, N, K, 1.0, self.d[0], M, self.d[1], K, 0.0,
+                           self.d[2], M)
+
+    def check(self):
+        torch.cuda.synchronize()
+        assert np.array_equal(self.d[2].download().reshape(self.want.shape), self.want)
+
+
+@pytest.fixture
+def stream_handle(built_lib):
+    st = torch.cuda.Stream()
+    s, h = hb.hcblasCreate(0, st.cuda_stream)
+    assert s == 0
+    yield h, st
+    hb.hcblasDestroy(h)
+
+
+def test_lowered_limit_holds_for_repeated_calls(stream_handle):
+    h, _ = stream_handle
+    assert hb.set_tuning(h, "graphs", 1) == 0
+    p = Product(1)
+    p.upload(h)
+    for limit, path in ((0, "tc.h."), (1, "simt.h."), (0, "tc.h.")):
+        assert hb.set_tuning(h, "workspace_mb", limit) == 0
+        for _ in range(3):
+            assert p.run(h) == 0
+            assert hb.hcblasGetLastPath(h).startswith(path), limit
+        p.check()
