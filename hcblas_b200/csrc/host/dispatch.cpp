@@ -69,6 +69,7 @@ int simt_f32_realigned(HcblasB200State *st, const hcbk_gemm_args *a, double us, 
   if (F32_ELEM_LOSS * us < 4.0 + 2.0 * (double)(bytes_a + bytes_b) / 4.2e6 ||
       a->k < 512 || bytes_a + bytes_b > REALIGN_F32_MAX)
     return HCBK_ERR_ALIGN;
+  const RelaxedCapture relaxed;
   char *ws = static_cast<char *>(call_scratch(st, bytes_a + bytes_b, stream));
   if (!ws) return HCBK_ERR_ALIGN;
   hcbk_gemm_args r = *a;
@@ -296,6 +297,7 @@ int hgemm_realigned(HcblasB200State *st, const hcbk_gemm_args *a, bool ok_a, boo
   auto up8 = [](int64_t v) { return (v + 7) & ~int64_t(7); };
   const size_t bytes_a = ok_a ? 0 : ((size_t)up8(in_a) * out_a * 2 + 255) & ~size_t(255);
   const size_t bytes_b = ok_b ? 0 : (size_t)up8(in_b) * out_b * 2;
+  const RelaxedCapture relaxed;
   char *ws = static_cast<char *>(call_scratch(st, bytes_a + bytes_b, stream));
   if (!ws) return HCBK_ERR_ALIGN;
   int *err = device_error_flag(st);

@@ -113,6 +113,14 @@ void *ensure_workspace(HcblasB200State *st, size_t bytes, void *stream_v) {
   return p;
 }
 
+RelaxedCapture::RelaxedCapture() : mode_(cudaStreamCaptureModeRelaxed) { swap(); }
+RelaxedCapture::~RelaxedCapture() { swap(); }
+void RelaxedCapture::swap() {
+  cudaStreamCaptureMode m = static_cast<cudaStreamCaptureMode>(mode_);
+  if (cudaThreadExchangeStreamCaptureMode(&m) != cudaSuccess) cudaGetLastError();
+  mode_ = (int)m;
+}
+
 static thread_local long long t_scratch_calls = 0;
 long long call_scratch_count() { return t_scratch_calls; }
 
@@ -172,14 +180,17 @@ void clear_graph_cache(HcblasB200State *st) {
 int *device_error_flag(HcblasB200State *st) {
   int dev = 0;
   cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> lock(st->scratch_mutex);
   if (st->dev_err && st->dev_err_device == dev) return st->dev_err;
+  const RelaxedCapture relaxed;
   if (st->dev_err) {
     clear_graph_cache(st);
     DeviceGuard g(st->dev_err_device);
     cudaFree(st->dev_err);
     st->dev_err = nullptr;
   }
-  /* the device error block: int 0 the code, ints 2-3 the wait limit (ns) */
+  /* the device error block: int 0 the code, ints 2-3 the wait limit (ns);
+   * written on a stream of its own, which waits for no other */
   void *p = nullptr;
   if (cudaMalloc(&p, 4 * sizeof(int)) != cudaSuccess) {
     cudaGetLastError();
@@ -187,7 +198,12 @@ int *device_error_flag(HcblasB200State *st) {
   }
   int block[4] = {0, 0, 0, 0};
   std::memcpy(block + 2, &st->wait_limit_ns, sizeof(st->wait_limit_ns));
-  if (cudaMemcpy(p, block, sizeof(block), cudaMemcpyHostToDevice) != cudaSuccess) {
+  cudaStream_t own = nullptr;
+  bool ok = cudaStreamCreateWithFlags(&own, cudaStreamNonBlocking) == cudaSuccess;
+  ok = ok && cudaMemcpyAsync(p, block, sizeof(block), cudaMemcpyHostToDevice, own) == cudaSuccess &&
+       cudaStreamSynchronize(own) == cudaSuccess;
+  if (own) cudaStreamDestroy(own);
+  if (!ok) {
     cudaGetLastError();
     cudaFree(p);
     return nullptr;

@@ -83,7 +83,8 @@ struct HcblasB200State {
   void *workspace_stream = nullptr; /* stream of the last call that used it */
   void *workspace_event = nullptr;  /* cudaEvent_t ordering a new stream after it */
   size_t workspace_limit = 0;       /* tuning knob "workspace_mb" (0 = none) */
-  /* per-device memory pools of call_scratch (created on first use) */
+  /* per-device memory pools of call_scratch (created on first use); the mutex
+   * also guards the device error block's creation */
   std::mutex scratch_mutex;
   void *scratch_pool[16] = {nullptr}; /* cudaMemPool_t */
   /* device error block of the tensor-core kernels: int 0 is set when a
@@ -171,6 +172,22 @@ class DeviceGuard {
  * `stream` is being captured, beyond the "workspace_mb" limit, or when the
  * allocation fails. */
 void *ensure_workspace(HcblasB200State *st, size_t bytes, void *stream);
+
+/* Set-up calls (allocations, pools, kernel attributes) while this thread or
+ * another captures some other stream in global mode: outside this scope they
+ * would invalidate that capture, which has nothing to do with the handle's own
+ * stream. */
+class RelaxedCapture {
+ public:
+  RelaxedCapture();
+  ~RelaxedCapture();
+  RelaxedCapture(const RelaxedCapture &) = delete;
+  RelaxedCapture &operator=(const RelaxedCapture &) = delete;
+
+ private:
+  void swap();
+  int mode_; /* cudaStreamCaptureMode of the thread outside */
+};
 
 /* Scratch memory of one call: allocated stream-ordered from the handle's own
  * pool and handed back with call_scratch_free after the call's last launch, so

@@ -51,3 +51,21 @@ def test_lowered_limit_holds_for_repeated_calls(stream_handle):
             assert p.run(h) == 0
             assert hb.hcblasGetLastPath(h).startswith(path), limit
         p.check()
+
+
+def test_capture_on_another_stream_goes_on(stream_handle):
+    """A handle's first call that copies its operands, while this thread captures
+    another stream in global mode: neither disturbs the other."""
+    h, _ = stream_handle
+    p = Product(4)
+    p.upload(h)
+    x = torch.zeros(1000, device="cuda")
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g, stream=torch.cuda.Stream(), capture_error_mode="global"):
+        x.add_(1)
+        assert p.run(h) == 0
+        x.add_(1)
+    g.replay()
+    p.check()
+    assert (x == 2).all()
