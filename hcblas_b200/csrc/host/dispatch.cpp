@@ -40,6 +40,9 @@ bool aligned16(const void *p, int64_t off, int esz) {
  * (beta != 0), 4095^3 3416 against 200.  Smaller products keep the path that needs neither scratch nor a second
  * launch. */
 constexpr double REALIGN_MIN_MNK = 268435456.0; /* 2^28 */
+/* the copies' size, what the scratch pool keeps: larger operands go through it
+ * in panels (8378 x 14522 pairs, the largest of ordinary calls, fit whole) */
+constexpr size_t REALIGN_H_MAX = (size_t)512 << 20;
 
 int simt_f32(HcblasB200State *st, const hcbk_gemm_args *a, void *stream, const char **path);
 
@@ -289,42 +292,56 @@ int hgemm_realigned(HcblasB200State *st, const hcbk_gemm_args *a, bool ok_a, boo
   if (st->inject_timeout || (double)a->m * (double)a->n * (double)a->k < REALIGN_MIN_MNK ||
       a->m > 0x7fffffff || a->n > 0x7fffffff || a->k > 0x7fffffff)
     return HCBK_ERR_ALIGN;
-  /* stored lines: `inner` contiguous elements, `outer` lines */
-  const int64_t in_a = a->op_a == HCBK_OP_N ? a->m : a->k;
-  const int64_t out_a = a->op_a == HCBK_OP_N ? a->k : a->m;
-  const int64_t in_b = a->op_b == HCBK_OP_N ? a->k : a->n;
-  const int64_t out_b = a->op_b == HCBK_OP_N ? a->n : a->k;
+  /* whole operands, or panels of M and N where their copies exceed the cap */
   auto up8 = [](int64_t v) { return (v + 7) & ~int64_t(7); };
-  const size_t bytes_a = ok_a ? 0 : ((size_t)up8(in_a) * out_a * 2 + 255) & ~size_t(255);
-  const size_t bytes_b = ok_b ? 0 : (size_t)up8(in_b) * out_b * 2;
+  const size_t budget = ok_a || ok_b ? REALIGN_H_MAX : REALIGN_H_MAX / 2;
+  auto panel = [&](bool in_place, int64_t rows) {
+    const int64_t most = (int64_t)(budget / 2 / (size_t)up8(a->k)) & ~int64_t(255);
+    return in_place || rows <= most ? rows : most;
+  };
+  const int64_t mp = panel(ok_a, a->m), np = panel(ok_b, a->n);
+  if (mp <= 0 || np <= 0) return HCBK_ERR_ALIGN; /* K alone exceeds it */
+  /* stored lines of a copy: `inner` contiguous elements, `outer` lines */
+  const bool a_mn = a->op_a == HCBK_OP_N, b_mn = a->op_b != HCBK_OP_N;
+  auto copy_bytes = [&](bool mn, int64_t rows) {
+    return (size_t)(mn ? up8(rows) * a->k : up8(a->k) * rows) * 2;
+  };
+  const size_t bytes_a = ok_a ? 0 : (copy_bytes(a_mn, mp) + 255) & ~size_t(255);
+  const size_t bytes_b = ok_b ? 0 : copy_bytes(b_mn, np);
   const RelaxedCapture relaxed;
   char *ws = static_cast<char *>(call_scratch(st, bytes_a + bytes_b, stream));
   if (!ws) return HCBK_ERR_ALIGN;
   int *err = device_error_flag(st);
-  if (!err) {
-    call_scratch_free(ws, stream);
-    return HCBK_ERR_ALIGN;
-  }
-  hcbk_gemm_args r = *a;
-  hcbk_realign_job jobs[2];
-  int count = 0;
-  if (!ok_a) {
-    jobs[count++] = {static_cast<const uint16_t *>(a->a) + a->a_off, a->lda, ws, up8(in_a),
-                     in_a, out_a};
-    r.a = ws;
-    r.a_off = 0;
-    r.lda = up8(in_a);
-  }
-  if (!ok_b) {
-    jobs[count++] = {static_cast<const uint16_t *>(a->b) + a->b_off, a->ldb, ws + bytes_a,
-                     up8(in_b), in_b, out_b};
-    r.b = ws + bytes_a;
-    r.b_off = 0;
-    r.ldb = up8(in_b);
-  }
-  int rc = timed_launch(st, stream, "pack.realign_f16",
-                        [&] { return hcbk_realign_f16(jobs, count, stream); });
-  if (!rc) rc = hgemm_tc_run(st, &r, true, err, stream, path);
+  int rc = err ? HCBK_OK : HCBK_ERR_ALIGN;
+  for (int64_t i0 = 0; !rc && i0 < a->m; i0 += mp)
+    for (int64_t j0 = 0; !rc && j0 < a->n; j0 += np) {
+      hcbk_gemm_args r = *a;
+      r.m = a->m - i0 < mp ? a->m - i0 : mp;
+      r.n = a->n - j0 < np ? a->n - j0 : np;
+      r.a_off += a_mn ? i0 : i0 * a->lda;
+      r.b_off += b_mn ? j0 : j0 * a->ldb;
+      r.c_off += i0 + j0 * a->ldc;
+      hcbk_realign_job jobs[2];
+      int count = 0;
+      auto operand = [&](bool mn, int64_t rows, const void *&src, int64_t &off, int64_t &ld,
+                         char *dst, bool copy) {
+        const int64_t inner = mn ? rows : a->k, outer = mn ? a->k : rows;
+        if (copy)
+          jobs[count++] = {static_cast<const uint16_t *>(src) + off, ld, dst, up8(inner), inner,
+                           outer};
+        src = dst;
+        off = 0;
+        ld = up8(inner);
+      };
+      if (!ok_a) operand(a_mn, r.m, r.a, r.a_off, r.lda, ws, j0 == 0);
+      if (!ok_b) operand(b_mn, r.n, r.b, r.b_off, r.ldb, ws + bytes_a, i0 == 0 || np < a->n);
+      if (count)
+        rc = timed_launch(st, stream, "pack.realign_f16",
+                          [&] { return hcbk_realign_f16(jobs, count, stream); });
+      if (!rc) rc = hgemm_tc_run(st, &r, true, err, stream, path);
+      /* C is partly done: no other path may start over */
+      if (i0 + j0 > 0 && rc) rc = HCBK_ERR_LAUNCH;
+    }
   call_scratch_free(ws, stream);
   return rc;
 }

@@ -527,9 +527,10 @@ hcblasStatus_t hcblasPlanEmulation(int mode, int param, int bits, int dtype, lon
  *                       fails the same way).
  *                       Native HGEMM (M N K >= 2^28) and SGEMM (K >= 512)
  *                       with operands off 16 bytes copy these into
- *                       stream-ordered scratch beside the workspace, from a
- *                       pool that keeps up to 512 MiB per device until the
- *                       handle is destroyed.  The limit holds for each call's
+ *                       stream-ordered scratch beside the workspace, at most
+ *                       512 MiB a call (HGEMM takes larger operands in panels,
+ *                       SGEMM in place), from a pool that keeps up to 512 MiB
+ *                       per device until the handle is destroyed.  The limit holds for each call's
  *                       copies by themselves; where they would exceed it,
  *                       while the stream is being captured, or without memory
  *                       the call runs more slowly on the operands in place

@@ -69,3 +69,40 @@ def test_capture_on_another_stream_goes_on(stream_handle):
     g.replay()
     p.check()
     assert (x == 2).all()
+
+
+@pytest.mark.parametrize("M,N", [(3400, 24), (24, 3400), (3400, 3401)])
+@pytest.mark.parametrize("ta,tb", [("n", "t"), ("t", "n")])
+def test_copies_above_the_cap_go_in_panels(handle, M, N, ta, tb):
+    """K = 40001: 3354 lines of either operand fill its half of the scratch."""
+    K = 40001
+    gen = torch.Generator(device="cuda").manual_seed(M + N)
+
+    class Dev:
+        dtype = np.dtype(np.float16)
+
+        def __init__(self, rows, cols):
+            self.t = torch.randint(-2, 3, (rows, cols), generator=gen, device="cuda").half()
+            self.ptr = self.t.data_ptr()
+
+    a = Dev(K, M + 1) if ta == "n" else Dev(M, K)  # lines of the column-major operands
+    b = Dev(N, K) if tb == "n" else Dev(K, N + 1)
+    c = Dev(N, M + 3)
+    want = c.t.clone()
+    A = a.t[:, :M].T if ta == "n" else a.t
+    B = b.t if tb == "n" else b.t[:, :N].T
+    prod = torch.zeros(N, M, device="cuda", dtype=torch.float64)
+    for k in range(0, K, 4096):  # exact: sums of integers
+        prod += B[:, k:k + 4096].double() @ A[:, k:k + 4096].double().T
+    want[:, :M] = (prod + 0.5 * c.t[:, :M].double()).half()
+    torch.cuda.synchronize()
+    hb.set_profiling(handle, True)
+    try:
+        assert hb.lib_gemm(handle, hb.ColMajor, ta, tb, M, N, K, 1.0, a, a.t.shape[1], b,
+                           b.t.shape[1], 0.5, c, M + 3) == 0
+        launches = hb.get_profile(handle)["pack.realign_f16"][0]
+    finally:
+        hb.set_profiling(handle, False)
+    assert hb.device_error(handle) == 0
+    assert launches == {24: 2, 3400: 4}[min(M, N)]
+    assert torch.equal(c.t, want)
