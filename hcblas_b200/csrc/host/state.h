@@ -192,7 +192,8 @@ class RelaxedCapture {
 /* Scratch memory of one call: allocated stream-ordered from the handle's own
  * pool and handed back with call_scratch_free after the call's last launch, so
  * calls on different streams (or from different threads) never share a buffer
- * and never wait for one another.  The pool keeps up to 512 MiB between calls
+ * at the same time; one waits for another's only where the device has no
+ * memory for a second.  The pool keeps up to 512 MiB between calls
  * and is given back with the handle.  nullptr while `stream` is being captured
  * (the memory would belong to the graph), beyond the "workspace_mb" limit, or
  * when the allocation fails: the caller then takes a path that needs no

@@ -53,6 +53,31 @@ def test_lowered_limit_holds_for_repeated_calls(stream_handle):
         p.check()
 
 
+def test_streams_do_not_wait_for_one_another(stream_handle):
+    """Scratch that a call on one stream has handed back is not taken on another
+    by waiting for the first."""
+    h, one = stream_handle
+    two = torch.cuda.Stream()
+    p, q = Product(2), Product(3)
+    p.upload(h)
+    q.upload(h)
+    torch.cuda._sleep(1000)
+    torch.cuda.synchronize()
+    busy, done = torch.cuda.Event(), torch.cuda.Event()
+    with torch.cuda.stream(one):
+        torch.cuda._sleep(4_000_000_000)  # about two seconds
+    assert p.run(h) == 0
+    busy.record(one)
+    assert hb.hcblasSetStream(h, two.cuda_stream) == 0
+    assert q.run(h) == 0
+    done.record(two)
+    done.synchronize()
+    assert not busy.query()
+    hb.hcblasSetStream(h, one.cuda_stream)
+    p.check()
+    q.check()
+
+
 def test_capture_on_another_stream_goes_on(stream_handle):
     """A handle's first call that copies its operands, while this thread captures
     another stream in global mode: neither disturbs the other."""
