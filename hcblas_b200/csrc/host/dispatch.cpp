@@ -34,11 +34,12 @@ bool aligned16(const void *p, int64_t off, int esz) {
 
 /* M N K from which HGEMM with operands that TMA cannot address copies them
  * into addressable scratch and runs on the tensor cores instead of the CUDA
- * cores.  Measured (B200, CUDA-core kernel against copy + tensor cores):
- * 645 x 645 x 647 37 against 17 us, 8378 x 32 x 1024 48 against 23,
- * 8191 x 4095 x 17 109 against 44, 8378 x 1133 x 777 521 against 51
- * (beta != 0), 4095^3 3416 against 200.  Smaller products keep the path that needs neither scratch nor a second
- * launch. */
+ * cores.  Measured at the line (B200, CUDA-core kernel against copy + tensor
+ * cores): 645 x 645 x 647 39 against 19 us, 1133 x 777 x 311 39 / 15, 2049 x
+ * 1027 x 129 39 / 17, 4095 x 4095 x 17 58 / 31, 131 x 130 x 16001 811 / 116;
+ * above it 1133 x 777 x 1133 123 / 21, 8378 x 1133 x 777 (beta != 0) 521 / 51,
+ * 4095^3 3416 / 200.  The line is not where the copy begins to pay (it halves
+ * the time there): smaller products keep the path that takes no scratch. */
 constexpr double REALIGN_MIN_MNK = 268435456.0; /* 2^28 */
 /* the copies' size, what the scratch pool keeps: larger operands go through it
  * in panels (8378 x 14522 pairs, the largest of ordinary calls, fit whole) */

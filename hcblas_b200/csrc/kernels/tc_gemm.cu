@@ -1405,14 +1405,16 @@ static int hgemm_tc_impl(const hcbk_gemm_args *a, int bn, int pair, int *err, vo
   }
   if (swap) {
     /* fewer stages: the columns' staging takes their place.  Eight epilogue
-     * warps where the epilogue bounds the tile, four where its MMAs do;
-     * measured (B200, CTA pairs): 8191 x 8191 x 33 93 against 130 us,
-     * 8378 x 1133 x 777 beta != 0 50 against 57, beta == 0 41 both,
-     * 4095^3 149 against 140. */
-    if (p.k <= (p.beta_nonzero ? 1024 : 512)) {
+     * warps where the epilogue bounds the tile: it reads C (beta != 0), the
+     * tile is 256 wide and K short; four and a stage more elsewhere.  Measured
+     * (B200, eight / four warps, us): 8191 x 8191 beta 0.5, pairs, K = 128 146 /
+     * 175, 1024 176 / 254, 2048 305 / 329, 4096 500 / 465; 128 x 256 tiles K =
+     * 1032 190 / 201, 4096 631 / 636; beta 0, pairs, K = 128 82 / 79, 1024 135 /
+     * 126; 128 x 128 tiles 2047 x 2047 x 512 beta 0.5 20.3 / 17.6, beta 0 14.5 /
+     * 12.8. */
+    if (bn == 256 && p.beta_nonzero && p.k <= 2048) {
       if (pair) return launch_cols<256, 4, EpiColsH<8>, 2>(p, stream);
-      if (bn == 256) return launch_cols<256, 3, EpiColsH<8>, 1>(p, stream);
-      return launch_cols<128, 4, EpiColsH<8>, 1>(p, stream);
+      return launch_cols<256, 3, EpiColsH<8>, 1>(p, stream);
     }
     if (pair) return launch_cols<256, 5, EpiColsH<4>, 2>(p, stream);
     if (bn == 256) return launch_cols<256, 3, EpiColsH<4>, 1>(p, stream);
