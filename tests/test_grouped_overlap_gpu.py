@@ -1,10 +1,14 @@
 """Grouped HGEMM calls queued without a wait: each call's table is built on the
 GPU in the memory of the last call's, and the product starts while the builder
-may still run."""
+may still run.  Entries of the longest lines."""
+import ctypes
+
 import numpy as np
 import pytest
 
 import hcblas_b200 as hb
+
+from tests.test_grouped_table_gpu import ENTRY, PROBLEM
 
 pytestmark = pytest.mark.gpu
 
@@ -48,3 +52,24 @@ def test_changing_problem_arrays(handle, count):
         for g, w in zip(play(False), want):
             assert np.array_equal(g, w)
     assert hb.device_error(handle) == 0
+
+
+@pytest.mark.parametrize("k", [(1 << 30) - 8, 1 << 30, (1 << 31) - 8])
+def test_entries_of_long_lines_match_encode(handle, k):
+    """op(A) is one line of k elements: 2 GiB and more of them."""
+    L = hb.lib()
+    i64, vp = ctypes.c_int64, ctypes.c_void_p
+    L.hcbk_grouped_encode.argtypes = [vp, ctypes.c_int, ctypes.c_int, i64, i64, i64, vp, i64, vp,
+                                      i64, vp, i64]
+    L.hcbk_grouped_build.argtypes = [vp, vp, vp, vp, ctypes.c_int, ctypes.c_int, vp]
+    table = hb.DeviceArray(handle, np.zeros(ENTRY, np.uint8))
+    desc = hb.DeviceArray(handle, np.zeros(4, np.int32))
+    at = 1 << 40  # an address only: nothing is read from it
+    e = (ctypes.c_uint8 * (ENTRY + 128))()
+    p = (ctypes.addressof(e) + 127) // 128 * 128
+    assert L.hcbk_grouped_encode(p, 1, 0, 1, 8, k, at, k, at, k, at + 2, 8) == 0
+    want = np.frombuffer((ctypes.c_uint8 * ENTRY).from_address(p), np.uint8)
+    prob = np.array([(at, at, at + 2, k, k, 8, 1, 8, k, 1, b"")], PROBLEM)  # 64-wide tiles
+    ts = np.array([0, 1], np.int32)
+    assert L.hcbk_grouped_build(prob.ctypes.data, ts.ctypes.data, table.ptr, desc.ptr, 1, 1, None) == 0
+    assert np.array_equal(table.download()[:256], want[:256])
