@@ -8,8 +8,7 @@
  * cores and through DMMA, but one m16n8k4 instruction does 512 multiply-adds
  * from 3 operand registers per lane where the CUDA-core form needs 16 DFMA
  * instructions and 32 register reads; the shared-memory traffic per flop
- * drops 4x, which leaves issue slots for loads and lets one CTA per SM keep
- * the FP64 pipe busy.
+ * drops 4x, which leaves issue slots for loads.
  *
  * Design: 64 x 64 CTA tiles, four CTAs of two warps per SM, each warp a
  * 64 x 32 block = 4 x 4 m16n8 accumulators (64 doubles per lane), multiplied
@@ -17,11 +16,11 @@
  * Small CTAs fill each other's ramps and barriers and waste less on edges and
  * the last wave than one CTA of eight warps on 128 x 128 (measured, B200:
  * 4096 x 4096 x 2048 NN 2149 against 2320 us, 8378 x 777 x 1133 531 / 870,
- * 2047 x 2047 x 333 TT 115 / 168, 3000 x 3000 x 32 35.2 / 37.3).  K advances in slabs of 16 through a ring of
- * shared-memory stages filled by cp.async (16-byte copies where the operand
- * is 16-byte aligned with an even leading dimension, 8-byte copies
- * otherwise; zero fill outside the matrix): an MN-contiguous operand is
- * kept as [k][mn], a K-contiguous one as [mn][k], so that each is copied
+ * 2047 x 2047 x 333 TT 115 / 168, 3000 x 3000 x 32 35.2 / 37.3).  K advances
+ * in slabs of 16 through a ring of shared-memory stages filled by cp.async
+ * (16-byte copies where the operand is 16-byte aligned with an even leading
+ * dimension, 8-byte copies otherwise; zero fill outside the matrix): an
+ * MN-contiguous operand is kept as [k][mn], a K-contiguous one as [mn][k], so that each is copied
  * along its contiguous dimension and the 16 lanes of a half-warp reading a
  * fragment hit 16 distinct bank pairs in either layout.  Few tiles: the CTAs
  * of a cluster share a tile's K and add up their partial tiles over the
@@ -401,7 +400,8 @@ __global__ void __launch_bounds__(DNT, DPER_SM) dmma_gemm_kernel(const __grid_co
  * 2 x 2, warp tiles 32 x 32 = 2 x 4 m16n8 accumulator pairs (one 128 x 64 tile
  * of 8 warps per SM: CN 2048 x 2048 x 512 710 us, two of 64 x 64 608; 3000 x
  * 300 x 100 47 and 41).  K advances in slabs of 16 complex elements through a
- * 2-stage ring filled by cp.async (the other CTA covers a slab's latency), one 16-byte copy per element (two 8-byte ones for an operand that is only
+ * 2-stage ring filled by cp.async (the other CTA covers a slab's latency), one
+ * 16-byte copy per element (two 8-byte ones for an operand that is only
  * 8-byte aligned), complex values kept interleaved: an MN-contiguous operand
  * as [k][mn] (pitch 66 elements), a K-contiguous one as
  * [mn][k] (pitch 20), so that each quarter-warp's 16-byte fragment loads --
@@ -435,7 +435,8 @@ struct ZmmaParams {
   int split; /* CTAs per tile (cluster size) */
 };
 
-/* one operand's slab of complex elements into a stage (see load_slab) */
+/* one operand's slab of complex elements into a stage: [k][mn] or [mn][k] as
+ * stored, one copy per element, zeros outside the matrix */
 template <bool MN, int ROWS, int NT>
 __device__ __forceinline__ void zload_slab(double2 *dst, const double2 *X, int64_t ld,
                                            int64_t rows, int64_t K, int64_t r0, int64_t k0,

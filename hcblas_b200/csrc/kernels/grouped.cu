@@ -3,12 +3,11 @@
  * problems (each its own M, N, K, transposes, leading dimensions and
  * pointers) in ONE launch.
  *
- * The host writes a device-side problem table (hcbk_grouped_entry: TMA
- * tensor maps of op(A) and op(B), the C block, the shape) and the prefix
- * sums of every problem's 128 x 128 tile count.  Each CTA (one per SM,
- * 192 threads) walks the global tile sequence t = blockIdx.x,
- * blockIdx.x + gridDim.x, ...; every role finds the tile's problem by a
- * binary search over the prefix sums:
+ * A table in device memory (hcbk_grouped_entry: TMA tensor maps of op(A) and
+ * op(B), the C block, the shape) and one descriptor per tile are written by a
+ * builder kernel ahead.  Each CTA (192 threads, one or two per SM) walks the
+ * global tile sequence t = blockIdx.x, blockIdx.x + gridDim.x, ...; every role
+ * loads the tile's descriptor:
  *   warp 0      TMA producer: A and B K-slabs of the tile's problem, through
  *               that problem's tensor maps (read from global memory), into a
  *               6-stage SW128 ring

@@ -73,8 +73,9 @@ typedef struct hcbk_simt_cfg {
  * accumulation.  Any op, ld, offset, alignment, batch. */
 int hcbk_gemm_simt(const hcbk_gemm_args *args, hcbk_simt_cfg cfg, void *stream);
 
-/* SGEMM / CGEMM on the FP32 FMA pipe: tile 0 = 128 x 128 floats (four warps),
- * 1 = 64 x 64 (one warp); split = CTAs of a cluster sharing a tile's K range
+/* SGEMM / CGEMM on the FP32 FMA pipe: tile 0 = 128 x 128 floats (eight warps;
+ * four for C and for S with both operands K-contiguous and aligned), 1 = 64 x
+ * 64 (two warps); split = CTAs of a cluster sharing a tile's K range
  * (1..8).  Any op, ld, offset, alignment, batch. */
 typedef struct hcbk_f32_cfg {
   int tile, split;
