@@ -865,6 +865,9 @@ __global__ void __launch_bounds__(64 + 32 * EpiWarps<EPI>::value, 1)
   const int nchunks = (kblocks + chunk_kb - 1) / chunk_kb;
   const int ntiles_local = tile0 < num_tiles ? (num_tiles - tile0 + tile_step - 1) / tile_step : 0;
   constexpr bool PAIRS = EPI::INPLACE && PROMOTE_KB > 0;
+  /* short chunks of one accumulator (EpiColsSumH): items without a division
+   * per chunk (1133 x 777 x 14521 156 -> 140 us; no gain elsewhere) */
+  constexpr bool STEP = PROMOTE_KB > 0 && EW == 8;
   const int nitems = ntiles_local * nchunks;
 
   if (warp == 0) {
@@ -875,16 +878,14 @@ __global__ void __launch_bounds__(64 + 32 * EpiWarps<EPI>::value, 1)
       bool ok = true;
       WorkItem w{tile0, -1, 0};
       TileMN tc_{0, 0};
-      int plane = 0;
       for (int i = 0; ok && i < nitems; ++i) {
-        if (PAIRS)
-          w = work_item(i, tile0, tile_step, ntiles_local, nchunks, PAIRS);
-        else
+        if constexpr (STEP)
           next_item(w, tile_step, nchunks);
-        if (PAIRS || w.c == 0) { /* a new tile */
-          plane = EPI::PLANE_BATCH ? w.t / tiles_per_plane : 0;
+        else
+          w = work_item(i, tile0, tile_step, ntiles_local, nchunks, PAIRS);
+        const int plane = EPI::PLANE_BATCH ? w.t / tiles_per_plane : 0;
+        if (!STEP || w.c == 0)
           tc_ = tile_mn(w.t - plane * tiles_per_plane, p.tiles_m, p.tiles_n);
-        }
         const int tm = tc_.m, tn = tc_.n;
         const int row0 = (tm * CG + (int)rank) * BM;               /* this CTA's A rows */
         const int col0 = tn * BN + (int)rank * (int)Cfg::B_ROWS;   /* this CTA's B rows */
@@ -992,10 +993,10 @@ __global__ void __launch_bounds__(64 + 32 * EpiWarps<EPI>::value, 1)
       WorkItem w{tile0, -1, 0};
       for (int i = 0; ok && i < nitems; ++i, ++ci) {
         {
-          if (PAIRS)
-            w = work_item(i, tile0, tile_step, ntiles_local, nchunks, PAIRS);
-          else
+          if constexpr (STEP)
             next_item(w, tile_step, nchunks);
+          else
+            w = work_item(i, tile0, tile_step, ntiles_local, nchunks, PAIRS);
           const int kc = w.c * chunk_kb;
           /* in-place mode: chunk c of a tile accumulates into its slot's
            * buffer on top of the epilogue's reduced value of chunk c - 1 */
