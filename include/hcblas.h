@@ -549,7 +549,10 @@ hcblasStatus_t hcblasPlanEmulation(int mode, int param, int bits, int dtype, lon
 hcblasStatus_t hcblasSetTuningParam(hcblasHandle_t handle, const char *name, int value);
 
 /* Extension: the path the last GEMM call on this handle took (a short static
- * string such as "simt.d.128x128" or "tc.h.256x256.pair"). */
+ * string such as "simt.d.128x128" or "tc.h.256x256.pair").  A name identifies a
+ * path of a type and stays with it: "dmma.d.128x128" and "dmma.z.128x64" are the
+ * FP64 tensor path, whose tiles are 64 x 64 now; ".k2", ".k4" and ".k8" say that
+ * the FP32 path shares each tile's K among that many blocks (up to 2, 4, 8). */
 const char *hcblasGetLastPath(hcblasHandle_t handle);
 
 /* Extension: library version string. */

@@ -40,16 +40,17 @@ def stream_handle(built_lib):
     hb.hcblasDestroy(h)
 
 
-def test_lowered_limit_holds_for_repeated_calls(stream_handle):
+@pytest.mark.parametrize("limits", [(0, 1, 0), (1, 0, 1)])
+def test_changed_limit_holds_for_repeated_calls(stream_handle, limits):
     h, _ = stream_handle
     assert hb.set_tuning(h, "graphs", 1) == 0
     p = Product(1)
     p.upload(h)
-    for limit, path in ((0, "tc.h."), (1, "simt.h."), (0, "tc.h.")):
+    for limit in limits:
         assert hb.set_tuning(h, "workspace_mb", limit) == 0
         for _ in range(3):
             assert p.run(h) == 0
-            assert hb.hcblasGetLastPath(h).startswith(path), limit
+            assert hb.hcblasGetLastPath(h).startswith("simt.h." if limit else "tc.h."), limit
         p.check()
 
 
