@@ -297,8 +297,9 @@ int hgemm_realigned(HcblasB200State *st, const hcbk_gemm_args *a, bool ok_a, boo
   auto up8 = [](int64_t v) { return (v + 7) & ~int64_t(7); };
   const size_t budget = ok_a || ok_b ? REALIGN_H_MAX : REALIGN_H_MAX / 2;
   auto panel = [&](bool in_place, int64_t rows) {
-    const int64_t most = (int64_t)(budget / 2 / (size_t)up8(a->k)) & ~int64_t(255);
-    return in_place || rows <= most ? rows : most;
+    const int64_t most = (int64_t)(budget / 2 / (size_t)up8(a->k));
+    /* whole tiles, or what a very long K leaves */
+    return in_place || rows <= most ? rows : most & (most >= 256 ? ~int64_t(255) : ~int64_t(7));
   };
   const int64_t mp = panel(ok_a, a->m), np = panel(ok_b, a->n);
   if (mp <= 0 || np <= 0) return HCBK_ERR_ALIGN; /* K alone exceeds it */

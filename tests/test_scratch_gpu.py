@@ -97,11 +97,13 @@ def test_capture_on_another_stream_goes_on(stream_handle):
     assert (x == 2).all()
 
 
-@pytest.mark.parametrize("M,N", [(3400, 24), (24, 3400), (3400, 3401)])
+@pytest.mark.parametrize("M,N,K,copies", [
+    (3400, 24, 40001, 2), (24, 3400, 40001, 2), (3400, 3401, 40001, 4),  # 3354 lines fit
+    (131, 130, 600001, 1), (300, 24, 1000001, 3),  # 223, 134 lines fit
+])
 @pytest.mark.parametrize("ta,tb", [("n", "t"), ("t", "n")])
-def test_copies_above_the_cap_go_in_panels(handle, M, N, ta, tb):
-    """K = 40001: 3354 lines of either operand fill its half of the scratch."""
-    K = 40001
+def test_copies_above_the_cap_go_in_panels(handle, M, N, K, copies, ta, tb):
+    """Either operand has half of the scratch, 256 MiB."""
     gen = torch.Generator(device="cuda").manual_seed(M + N)
 
     class Dev:
@@ -130,5 +132,5 @@ def test_copies_above_the_cap_go_in_panels(handle, M, N, ta, tb):
     finally:
         hb.set_profiling(handle, False)
     assert hb.device_error(handle) == 0
-    assert launches == {24: 2, 3400: 4}[min(M, N)]
+    assert launches == copies
     assert torch.equal(c.t, want)
